@@ -54,10 +54,10 @@ int launch_stage_brick_hybrid(const Grid &, const ModelParams &, const StageArgs
 int launch_stage_march_fast(const Grid &, const ModelParams &, const StageArgs &, int, bool, int, cudaStream_t);
 int launch_stage_march_fp32(const Grid &, const ModelParams &, const StageArgs &, int, bool, bool, int,
                             cudaStream_t);
-int launch_stage_plane_fast(const Grid &, const ModelParams &, const StageArgs &, int, bool, const PlaneTile &,
-                            const CUtensorMap &, cudaStream_t);
 int launch_stage_plane_fp32(const Grid &, const ModelParams &, const StageArgs &, int, bool, bool,
                             const PlaneTile &, const CUtensorMap &, cudaStream_t);
+int launch_stage_line(const Grid &, const ModelParams &, const StageArgs &, int, bool, const LineTile &,
+                      const CUtensorMap &, const CUtensorMap &, cudaStream_t);
 int launch_weno_batch_exact(int, const double *, double *, int, cudaStream_t);
 int launch_weno_batch_fast(int, const double *, double *, int, cudaStream_t);
 int launch_weno_batch_fp32(int, const double *, double *, int, cudaStream_t);
@@ -100,13 +100,15 @@ bool pdl_enabled()
 // Stage-kernel variants: the brick tile shapes (0 .. kTileVariants-1), the
 // line-march kernels and the plane-march kernels, each launched with 1, 2 or
 // 4 waves; the plane march twice: lines cut into equal segments per tile,
-// then equal shares of all tiles' planes per block
+// then equal shares of all tiles' planes per block.  The plane variants of the
+// FP64 form run the kernels of sweep_line.cuh.
 constexpr int kMarchVariants = 3;
 constexpr int kMarchWaves[kMarchVariants] = {1, 2, 4};
 constexpr int kPlaneVariants = 6;
 constexpr int kPlaneWaves[kPlaneVariants] = {1, 2, 4, 1, 2, 4};
 constexpr bool kPlaneShare[kPlaneVariants] = {false, false, false, true, true, true};
 constexpr int kPlaneFirst = kTileVariants + kMarchVariants;
+constexpr long long kLineDefaultNodes = 1 << 18;  // computed nodes (acfd_init)
 constexpr int kStageVariants = kPlaneFirst + kPlaneVariants;
 static_assert(ACFD_BRICK_VARIANTS == kTileVariants && ACFD_STAGE_VARIANTS == kStageVariants &&
                   ACFD_PLANE_VARIANT == kPlaneFirst,
@@ -126,6 +128,14 @@ using namespace acfd;
 struct StepPiece {
     int kind, axis, stage;
     cudaEvent_t e0, e1;
+};
+
+// tensor maps of the FP64 line march along one axis: a plane of U[tn] with
+// its halo and the tile's plane of U[to], with the extents they were encoded for
+struct LineMaps {
+    CUtensorMap map, omap;
+    int BXp = 0, BC = 0, OX = 0, NR = 0;
+    bool ok = false;
 };
 
 struct acfd_case {
@@ -170,6 +180,8 @@ struct acfd_case {
     CUtensorMap pmaps[3];          // plane-march state maps per sweep axis
     int pbox[3][2] = {{0, 0}, {0, 0}, {0, 0}};  // their box: x extent and rows
     bool pmaps_ok = false;
+    LineMaps line[3];              // FP64 line march: maps per sweep axis ...
+    LineMaps xline;                // ... and of the Y sweep of the transposed state
     bool plain_kernels = false;    // use the global-memory stage kernels instead of the bricks
     bool bc_multi = false;         // one launch per ghost-fill phase instead of the fused launch
     unsigned *bcbar = nullptr;     // grid-barrier words of the fused ghost fill
@@ -245,9 +257,9 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
     return encode;
 }
 
-// map of the whole state of a case with the given box (x, y, z), five
+// map of the whole state of a case with the given box (x, y, z), nvar
 // variables, one level
-int encode_box_map(const Grid &g, double *U, const int b[3], CUtensorMap *out)
+int encode_box_map(const Grid &g, double *U, const int b[3], CUtensorMap *out, int nvar = kVars)
 {
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (!encode) {
@@ -257,7 +269,7 @@ int encode_box_map(const Grid &g, double *U, const int b[3], CUtensorMap *out)
     const cuuint64_t strides[4] = {(cuuint64_t)g.pitch * 8, (cuuint64_t)g.pitch * g.n[1] * 8,
                                    (cuuint64_t)g.nn * 8, (cuuint64_t)g.nn * 5 * 8};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    const cuuint32_t box[5] = {(cuuint32_t)b[0], (cuuint32_t)b[1], (cuuint32_t)b[2], 5, 1};
+    const cuuint32_t box[5] = {(cuuint32_t)b[0], (cuuint32_t)b[1], (cuuint32_t)b[2], (cuuint32_t)nvar, 1};
     CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 5, U, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -266,6 +278,40 @@ int encode_box_map(const Grid &g, double *U, const int b[3], CUtensorMap *out)
         return ACFD_ERR_CUDA;
     }
     return ACFD_OK;
+}
+
+// maps of the line march of sweep s over the state U of grid g;
+// maps.ok stays false where no tile fits
+int encode_line_maps(const Grid &g, double *U, int s, bool visc, int sms, LineMaps &maps)
+{
+    const LineTile lt = line_tile(g, s, visc, 1, sms, true);
+    if (lt.pt.NR < 1 || lt.pt.BC > 256) {
+        return ACFD_OK;
+    }
+    const int box[3] = {lt.pt.BXp, s == 2 ? lt.pt.BC : 1, s == 2 ? 1 : lt.pt.BC};
+    const int obox[3] = {lt.OX, s == 2 ? lt.pt.NR : 1, s == 2 ? 1 : lt.pt.NR};
+    int st = encode_box_map(g, U, box, &maps.map, 1);
+    if (st == ACFD_OK) st = encode_box_map(g, U, obox, &maps.omap, 1);
+    if (st != ACFD_OK) return st;
+    maps.BXp = lt.pt.BXp;
+    maps.BC = lt.pt.BC;
+    maps.OX = lt.OX;
+    maps.NR = lt.pt.NR;
+    maps.ok = true;
+    return ACFD_OK;
+}
+
+// one FP64 stage on the line march, the launch cut as plane variant v asks
+int line_stage(const acfd_case *cs, const Grid &g, const StageArgs &a, int s, int v, const LineMaps &maps)
+{
+    const bool visc = viscous(cs);
+    const LineTile lt = line_tile(g, s, visc, kPlaneWaves[v - kPlaneFirst], cs->sms, kPlaneShare[v - kPlaneFirst]);
+    if (!maps.ok || lt.pt.BXp != maps.BXp || lt.pt.BC != maps.BC || lt.OX != maps.OX || lt.pt.NR != maps.NR) {
+        set_error("line tile (%d x %d) does not match its encoded box (%d x %d)", lt.pt.BXp, lt.pt.BC, maps.BXp,
+                  maps.BC);
+        return ACFD_ERR_STATE;
+    }
+    return launch_stage_line(g, cs->mp, a, s, visc, lt, maps.map, maps.omap, cs->stream);
 }
 
 int encode_state_maps(acfd_case *cs)
@@ -315,6 +361,10 @@ int encode_state_maps(acfd_case *cs)
         }
     }
     cs->pmaps_ok = true;
+    for (int s = 0; s < 3; ++s) {
+        const int st = encode_line_maps(g, cs->U, s, viscous(cs), cs->sms, cs->line[s]);
+        if (st != ACFD_OK) return st;
+    }
     return ACFD_OK;
 }
 
@@ -684,6 +734,7 @@ void build_xt(acfd_case *cs)
     cs->xbox[0] = pt.BXp;
     cs->xbox[1] = pt.BC;
     cs->xg = xg;
+    if (cs->xt_all_forms && encode_line_maps(xg, cs->xU, 1, viscous(cs), cs->sms, cs->xline) != ACFD_OK) return;
     if (launch_transpose_int(cs->flags, g, cs->xdid, xg, cs->stream) != ACFD_OK) return;
     cs->xt_ok = true;
 }
@@ -819,7 +870,7 @@ int stage(acfd_case *cs, double dt_scale, double coeA, double coeB, int to, int 
         const int waves = plane_v ? kPlaneWaves[var - kPlaneFirst] : march ? kMarchWaves[var - kTileVariants] : 1;
         const int target32 = waves * cs->sms * 16, target64 = waves * cs->sms * 8;
         PlaneTile pt = {};
-        if (plane) {
+        if (plane && cs->mode != ACFD_FP64) {
             pt = plane_tile(cs->grid, s, visc, waves, cs->sms, kPlaneShare[var - kPlaneFirst]);
             if (pt.BXp != cs->pbox[s][0] || pt.BC != cs->pbox[s][1]) {
                 set_error("plane tile (%d x %d) does not match the encoded box (%d x %d) of axis %d", pt.BXp, pt.BC,
@@ -830,7 +881,7 @@ int stage(acfd_case *cs, double dt_scale, double coeA, double coeB, int to, int 
         switch (cs->mode) {
             case ACFD_FP64_EXACT: st = launch_stage_exact(cs->grid, cs->mp, a, s, visc, cs->stream); break;
             case ACFD_FP64:
-                st = plane   ? launch_stage_plane_fast(cs->grid, cs->mp, a, s, visc, pt, cs->pmaps[s], cs->stream)
+                st = plane   ? line_stage(cs, cs->grid, a, s, var, cs->line[s])
                      : march ? launch_stage_march_fast(cs->grid, cs->mp, a, s, visc, target64, cs->stream)
                      : brick ? launch_stage_brick_fast(cs->grid, cs->mp, a, s, visc, cs->stream)
                              : launch_stage_fast(cs->grid, cs->mp, a, s, visc, cs->stream);
@@ -926,7 +977,7 @@ int discretize(acfd_case *cs, double dt_scale, int s)
 bool xt_eligible(const acfd_case *cs)
 {
     const bool form = cs->mode == ACFD_FP32_HYBRID || cs->mode == ACFD_FP32_BULK ||
-                      (cs->xt_all_forms && cs->mode != ACFD_FP64_EXACT);
+                      (cs->xt_all_forms && cs->mode == ACFD_FP64 && cs->xline.ok);
     return cs->xt_ok && !cs->debug && !cs->plain_kernels && form && !(cs->ib && ib_count(cs->ib) > 0);
 }
 
@@ -978,7 +1029,7 @@ int stage_xt(acfd_case *cs, double dt_scale, double coeA, double coeB, int to, i
     }
     int st;
     switch (cs->mode) {
-        case ACFD_FP64: st = launch_stage_plane_fast(cs->xg, cs->mp, a, 1, visc, pt, cs->xmap, cs->stream); break;
+        case ACFD_FP64: st = line_stage(cs, cs->xg, a, 1, var, cs->xline); break;
         case ACFD_FP32_HYBRID:
             st = launch_stage_plane_fp32(cs->xg, cs->mp, a, 1, visc, true, pt, cs->xmap, cs->stream);
             break;
@@ -1358,6 +1409,13 @@ int acfd_init(const acfd_partition_t *part, const acfd_model_t *model, acfd_case
     }
     g.pitch = (part->n[0] + 7) & ~7;
     g.nn = (long long)g.pitch * g.n[1] * g.n[2];
+    // the FP64 form starts on the line march with equal shares where it is
+    // faster than the brick: step times on the brick and the line march, us:
+    // 33^3 nodes 211 / 566, 96x62x34 (WENO3) 310 / 373, 65^3 656 / 641,
+    // 158x96x60 1,558 / 1,356, 7.1 M nodes around bodies 11,415 / 8,675
+    if ((long long)(g.hi[0] - g.lo[0]) * (g.hi[1] - g.lo[1]) * (g.hi[2] - g.lo[2]) >= kLineDefaultNodes) {
+        for (int s = 0; s < 3; ++s) cs->tile_var[ACFD_FP64][s] = kPlaneFirst + 3;
+    }
     ModelParams &m = cs->mp;
     m.gamma = model->gamma;
     m.gasR = model->gasR;

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
+
 #include "acfd.h"
 #include "launch.cuh"
 
@@ -197,6 +199,103 @@ inline PlaneTile plane_tile(const Grid &g, int s, bool visc, int waves, int sms,
 inline int plane_smem_bytes(const PlaneTile &pt, int s)
 {
     return plane_smem_total(pt.BXp, pt.BC, s == 0 ? pt.TR * pt.NR : 0, pt.ncw);
+}
+
+// Line-march kernels of the FP64 form (sweep_line.cuh): one block per SM, eight
+// consumer warps (two per scheduler) and a producer's warpgroup.  The ring holds
+// planes of U[tn] and kLineOSlots tiles of U[to], each variable at a fixed
+// stride (one copy per variable), so that the kernel's shared-memory addresses
+// are immediate offsets.
+constexpr int kLineWarps = 8;
+constexpr int kLineThreads = (kLineWarps + 4) * 32;
+// launched with 384 x 168 registers: 256 x 232 + 128 x 40
+constexpr int kLineConsumerRegs = 232, kLineProducerRegs = 40;
+constexpr int kLinePlane = 368, kLineOPlane = 272;  // elements of a variable in a slot (128-byte multiples)
+constexpr int kLineOSlots = 4;
+
+// slots of U[tn]: the planes of the stencil and those on their way (at most
+// np - 1 + kLineOSlots on Y and Z sweeps, 2 hv + kLineOSlots on X sweeps: see
+// the producers)
+__host__ __device__ constexpr int line_slots(int np)
+{
+    return np - 1 + kLineOSlots;
+}
+__host__ __device__ constexpr int line_x_slots(bool visc)
+{
+    return (visc ? 2 : 0) + kLineOSlots;
+}
+__host__ __device__ constexpr int line_smem_bytes(int slots)
+{
+    return slots * (5 * kLinePlane * 8 + 2 * 8) + kLineOSlots * 5 * kLineOPlane * 8;
+}
+static_assert(line_smem_bytes(line_slots(6)) <= 227 * 1024, "shared memory of a block");
+
+struct LineTile {
+    PlaneTile pt;
+    int OX;  // x extent of the tile of U[to] (even)
+};
+
+// Tile of the line march of sweep s: of the widths whose planes fit, the one
+// that leaves the fewest consumer lanes without a line, the halo's share of the
+// planes counting a tenth; then the cuts of plane_tile with one block per SM.
+// X sweeps place WX + 2 nodes of a row in the warps, 30 of a warp's 32 lanes
+// counting (stage_line_x).
+inline LineTile line_tile(const Grid &g, int s, bool visc, int waves, int sms, bool share)
+{
+    LineTile best = {};
+    const int T2 = (s == 2) ? 1 : 2, M = (s == 0) ? 1 : s;
+    const int Lx = g.hi[0] - g.lo[0], Lt = g.hi[T2] - g.lo[T2], Ls = g.hi[M] - g.lo[M];
+    const int hv = visc ? 1 : 0, hx = (s == 0) ? 3 : hv;
+    const int lines = (s == 0) ? kLineWarps * 30 + 2 : kLineWarps * 32, per_row = (s == 0) ? 2 : 0;
+    double cost = -1.0;
+    for (int ntx = 1; ntx <= (Lx > 0 ? Lx : 1); ++ntx) {
+        LineTile lt = {};
+        PlaneTile &pt = lt.pt;
+        pt.ntx = ntx;
+        pt.WX = (Lx + ntx - 1) / ntx;
+        if (pt.WX < 1) pt.WX = 1;
+        pt.TR = pt.WX + per_row;
+        pt.BXp = (pt.WX + 2 * hx + 2) & ~1;
+        lt.OX = (pt.WX + 2) & ~1;
+        if (pt.BXp > 256) continue;
+        if (cost >= 0.0 && pt.WX < 12) break;
+        pt.NR = std::min(std::min(lines / pt.TR, Lt), std::min(kLinePlane / pt.BXp - 2 * hv, kLineOPlane / lt.OX));
+        if (pt.NR < 1) continue;
+        pt.BC = pt.NR + 2 * hv;
+        pt.ntc = (Lt + pt.NR - 1) / pt.NR;
+        pt.ncw = kLineWarps;
+        const double c = (double)pt.ntx * pt.ntc * (kLineWarps * 32 + 0.1 * pt.BXp * pt.BC);
+        if (cost < 0.0 || c < cost) {
+            best = lt;
+            cost = c;
+        }
+    }
+    PlaneTile &pt = best.pt;
+    if (cost < 0.0) return best;
+    const long long tiles = (long long)pt.ntx * pt.ntc, target = (long long)waves * sms;
+    const int cap = Ls / 8 > 1 ? Ls / 8 : 1;
+    pt.share = share ? 1 : 0;
+    if (!share) {
+        pt.nseg = (int)std::max<long long>(1, std::min<long long>((target + tiles - 1) / tiles, cap));
+        if (waves == 1) {
+            // the fewest iterations: a segment of n planes takes n + 1, and
+            // about two more while its ring fills (small grids are cut below
+            // eight planes where the chip would idle)
+            long long least = 0;
+            for (int n = 1; n <= Ls; ++n) {
+                const long long it = (tiles * n + sms - 1) / sms * ((Ls + n - 1) / n + 3);
+                if (n == 1 || it < least) {
+                    least = it;
+                    pt.nseg = n;
+                }
+            }
+        }
+        pt.nblk = (int)(tiles * pt.nseg);
+    } else {
+        pt.nblk = (int)std::max<long long>(1, std::min<long long>(target, tiles * Ls / 8));
+        pt.nseg = (int)std::max<long long>(1, std::min<long long>((pt.nblk + tiles / 2) / tiles, cap));
+    }
+    return best;
 }
 
 // plane-march geometry of one case and sweep axis of a batch: the kernel's

@@ -48,14 +48,14 @@ int launch_stage_march_fast(const Grid &g, const ModelParams &m, const StageArgs
 
 }  // namespace acfd
 
-#include "sweep_plane.cuh"
+#include "sweep_line.cuh"
 
 namespace acfd {
 
-int launch_stage_plane_fast(const Grid &g, const ModelParams &m, const StageArgs &a, int s, bool viscous,
-                            const PlaneTile &pt, const CUtensorMap &map, cudaStream_t st)
+int launch_stage_line(const Grid &g, const ModelParams &m, const StageArgs &a, int s, bool viscous, const LineTile &lt,
+                      const CUtensorMap &map, const CUtensorMap &omap, cudaStream_t st)
 {
-    return form_fast::launch_plane_impl(g, m, a, s, viscous, false, pt, map, st);
+    return form_fast::launch_line_impl(g, m, a, s, viscous, lt, map, omap, st);
 }
 
 }  // namespace acfd
