@@ -15,8 +15,8 @@
 // characteristic fluxes (Roe average, LLF splitting).  A node is non-smooth
 // where it exceeds the training threshold.
 //
-// Kernels: feature/label extraction, MLP forward, MLP loss gradient (one
-// thread per sample, warp-reduced into shared then global accumulators),
+// Kernels: feature/label extraction, MLP forward, MLP loss gradient (tiles of
+// 64 samples in shared memory, the weight gradients as products over the tile),
 // Adam update, and flag inference for the three sweep axes: a pass that
 // stores (rho, p) of every node as float2, then a warp-per-32-nodes pass that
 // runs layers 1 and 2 as f16 tensor-core MMAs with f32 accumulation.
@@ -218,67 +218,197 @@ __device__ __forceinline__ float warp_sum(float v)
 // gradient: loss = w*(softplus(z) - y*z), dL/dz = w*(sigmoid(z) - y), with
 // w = pos_weight for y = 1.  grad and loss are accumulated (the caller
 // zeroes them).
-__global__ void __launch_bounds__(256) mlp_grad_kernel(const float *params, const float *X, const float *Y, int n,
-                                                       float pos_weight, float *grad, float *loss)
+//
+// A block takes tiles of 64 samples.  Every layer is a small product over the
+// tile in shared memory (rows of one hidden unit, kRow floats apart so that
+// float4 reads of consecutive rows do not collide): thread (s, rg) computes the
+// units 8 rg .. 8 rg + 7 of sample s forward and backward, then the weight
+// gradients -- sums over the samples -- are products of the stored rows, a
+// 2 x 2 patch of dW2 per thread, all in FP32.  The sums stay in registers over a
+// block's tiles and reach memory in one atomic per parameter and block.  What
+// bounds it is the latency of its six phases (16,384 samples: 256 blocks of one
+// tile); a warp reduction per weight and warp, with one thread per sample, took
+// 395 us for 16,384 samples.
+constexpr int kTile = 64, kRow = kTile + 4, kGradThreads = 256;
+constexpr int kGradBlocks = 2 * 148;
+
+__device__ __forceinline__ float sum8(float v)
 {
-    __shared__ float P[kParams];
-    __shared__ float G[kParams];
-    for (int q = threadIdx.x; q < kParams; q += blockDim.x) {
-        P[q] = params[q];
-        G[q] = 0.0f;
-    }
-    __syncthreads();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = t < n;
-    float x[kIn], h1[kH], h2[kH];
-#pragma unroll
-    for (int q = 0; q < kIn; ++q) x[q] = valid ? X[(long long)t * kIn + q] : 0.0f;
-    const float z = mlp_logit(P, x, h1, h2);
-    const float y = valid ? Y[t] : 0.0f;
-    const float w = valid ? (y > 0.5f ? pos_weight : 1.0f) : 0.0f;
-    const float sp = (z > 0.0f) ? z + log1pf(expf(-z)) : log1pf(expf(z));
-    const float l = w * (sp - y * z);
-    const float dz = w * (1.0f / (1.0f + expf(-z)) - y);
-    const int lane = threadIdx.x & 31;
-    // layer 3
-    float s = warp_sum(dz);
-    if (lane == 0) atomicAdd(&G[oB3], s);
-    float d2[kH];
-#pragma unroll
-    for (int q = 0; q < kH; ++q) {
-        s = warp_sum(dz * h2[q]);
-        if (lane == 0) atomicAdd(&G[oW3 + q], s);
-        d2[q] = (h2[q] > 0.0f) ? dz * P[oW3 + q] : 0.0f;
-    }
-    // layer 2
-    float d1[kH];
-#pragma unroll
-    for (int q = 0; q < kH; ++q) d1[q] = 0.0f;
-    for (int a = 0; a < kH; ++a) {
-        s = warp_sum(d2[a]);
-        if (lane == 0) atomicAdd(&G[oB2 + a], s);
-#pragma unroll
-        for (int q = 0; q < kH; ++q) {
-            s = warp_sum(d2[a] * h1[q]);
-            if (lane == 0) atomicAdd(&G[oW2 + a * kH + q], s);
-            d1[q] = fmaf(d2[a], P[oW2 + a * kH + q], d1[q]);
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    v += __shfl_xor_sync(0xffffffffu, v, 2);
+    v += __shfl_xor_sync(0xffffffffu, v, 4);
+    return v;
+}
+
+__device__ __forceinline__ float dot4(float4 a, float4 b, float c)
+{
+    return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c))));
+}
+
+__global__ void __launch_bounds__(kGradThreads) mlp_grad_kernel(const float *params, const float *X, const float *Y,
+                                                                int n, float pos_weight, float *grad, float *loss)
+{
+    __shared__ __align__(16) float P[(kParams + 3) / 4 * 4];
+    __shared__ __align__(16) float sX[kIn * kRow], sH1[kH * kRow], sD2[kH * kRow];
+    __shared__ __align__(16) float sQ[kH * kRow];  // H2, then D1
+    __shared__ __align__(16) float sdz[kTile];
+    __shared__ float sz[4][kTile];
+    const int tid = threadIdx.x;
+    for (int q = tid; q < kParams; q += kGradThreads) P[q] = params[q];
+    const int s = tid & (kTile - 1), rg = tid / kTile, r0 = 8 * rg;  // sample, first unit
+    const int row = tid >> 3, part = tid & 7;                        // bias and w3 sums
+    const int a0 = tid >> 4, q0 = tid & 15;                          // dW2: rows a0, a0 + 16, columns q0, q0 + 16
+    float g2[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}}, g1[2] = {0.0f, 0.0f};
+    float gb1 = 0.0f, gb2 = 0.0f, gw3 = 0.0f, gb3 = 0.0f, gl = 0.0f;
+    const long long tiles = ((long long)n + kTile - 1) / kTile;
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const long long first = tile * kTile;
+        const int m = (int)min((long long)kTile, n - first);  // samples of the tile
+        __syncthreads();
+        for (int q = tid; q < kTile * kIn; q += kGradThreads) {
+            const int i = q / kIn;
+            sX[(q - i * kIn) * kRow + i] = i < m ? X[first * kIn + q] : 0.0f;
         }
-    }
-    // layer 1
-    for (int a = 0; a < kH; ++a) {
-        const float da = (h1[a] > 0.0f) ? d1[a] : 0.0f;
-        s = warp_sum(da);
-        if (lane == 0) atomicAdd(&G[oB1 + a], s);
+        __syncthreads();
+        // layer 1
+        float h1[8], h2[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) h1[r] = P[oB1 + r0 + r];
 #pragma unroll
         for (int q = 0; q < kIn; ++q) {
-            s = warp_sum(da * x[q]);
-            if (lane == 0) atomicAdd(&G[oW1 + a * kIn + q], s);
+            const float x = sX[q * kRow + s];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) h1[r] = fmaf(P[oW1 + (r0 + r) * kIn + q], x, h1[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            h1[r] = fmaxf(h1[r], 0.0f);
+            sH1[(r0 + r) * kRow + s] = h1[r];
+            h2[r] = P[oB2 + r0 + r];
+        }
+        __syncthreads();
+        // layer 2 and this thread's share of the output layer
+#pragma unroll 2
+        for (int q = 0; q < kH; q += 4) {
+            const float x0 = sH1[q * kRow + s], x1 = sH1[(q + 1) * kRow + s];
+            const float x2 = sH1[(q + 2) * kRow + s], x3 = sH1[(q + 3) * kRow + s];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const float4 w = *reinterpret_cast<const float4 *>(P + oW2 + (r0 + r) * kH + q);
+                h2[r] = fmaf(w.w, x3, fmaf(w.z, x2, fmaf(w.y, x1, fmaf(w.x, x0, h2[r]))));
+            }
+        }
+        float z = 0.0f;
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            h2[r] = fmaxf(h2[r], 0.0f);
+            sQ[(r0 + r) * kRow + s] = h2[r];
+            z = fmaf(P[oW3 + r0 + r], h2[r], z);
+        }
+        sz[rg][s] = z;
+        __syncthreads();
+        if (tid < kTile) {
+            const bool valid = s < m;
+            const float zz = P[oB3] + ((sz[0][s] + sz[1][s]) + (sz[2][s] + sz[3][s]));
+            const float y = valid ? Y[first + s] : 0.0f;
+            const float w = valid ? (y > 0.5f ? pos_weight : 1.0f) : 0.0f;
+            const float ex = expf(-fabsf(zz));
+            const float sp = fmaxf(zz, 0.0f) + log1pf(ex);
+            const float sg = zz >= 0.0f ? 1.0f / (1.0f + ex) : ex / (1.0f + ex);
+            const float dz = w * (sg - y);
+            sdz[s] = dz;
+            gl += w * (sp - y * zz);
+            gb3 += dz;
+        }
+        __syncthreads();
+        {
+            const float dz = sdz[s];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                sD2[(r0 + r) * kRow + s] = h2[r] > 0.0f ? dz * P[oW3 + r0 + r] : 0.0f;
+            }
+            // w3: eight samples a thread of this thread's row
+            const float4 *h = reinterpret_cast<const float4 *>(sQ + row * kRow + 8 * part);
+            const float4 *d = reinterpret_cast<const float4 *>(sdz + 8 * part);
+            gw3 += sum8(dot4(h[0], d[0], dot4(h[1], d[1], 0.0f)));
+        }
+        __syncthreads();
+        // layer 2 backward: D1 = (W2^T D2) where layer 1 is active
+        float d1[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) d1[r] = 0.0f;
+#pragma unroll 4
+        for (int a = 0; a < kH; ++a) {
+            const float d = sD2[a * kRow + s];
+            const float4 w0 = *reinterpret_cast<const float4 *>(P + oW2 + a * kH + r0);
+            const float4 w1 = *reinterpret_cast<const float4 *>(P + oW2 + a * kH + r0 + 4);
+            d1[0] = fmaf(w0.x, d, d1[0]);
+            d1[1] = fmaf(w0.y, d, d1[1]);
+            d1[2] = fmaf(w0.z, d, d1[2]);
+            d1[3] = fmaf(w0.w, d, d1[3]);
+            d1[4] = fmaf(w1.x, d, d1[4]);
+            d1[5] = fmaf(w1.y, d, d1[5]);
+            d1[6] = fmaf(w1.z, d, d1[6]);
+            d1[7] = fmaf(w1.w, d, d1[7]);
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) sQ[(r0 + r) * kRow + s] = h1[r] > 0.0f ? d1[r] : 0.0f;
+        // dW2 and the bias of layer 2 (D2 and H1 are complete)
+        for (int t = 0; t < kTile; t += 4) {
+            const float4 u0 = *reinterpret_cast<const float4 *>(sD2 + a0 * kRow + t);
+            const float4 u1 = *reinterpret_cast<const float4 *>(sD2 + (a0 + 16) * kRow + t);
+            const float4 v0 = *reinterpret_cast<const float4 *>(sH1 + q0 * kRow + t);
+            const float4 v1 = *reinterpret_cast<const float4 *>(sH1 + (q0 + 16) * kRow + t);
+            g2[0][0] = dot4(u0, v0, g2[0][0]);
+            g2[0][1] = dot4(u0, v1, g2[0][1]);
+            g2[1][0] = dot4(u1, v0, g2[1][0]);
+            g2[1][1] = dot4(u1, v1, g2[1][1]);
+        }
+        const float4 one = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+        {
+            const float4 *d = reinterpret_cast<const float4 *>(sD2 + row * kRow + 8 * part);
+            gb2 += sum8(dot4(d[0], one, dot4(d[1], one, 0.0f)));
+        }
+        __syncthreads();
+        // dW1 and the bias of layer 1
+        {
+            const float4 *d = reinterpret_cast<const float4 *>(sQ + row * kRow + 8 * part);
+            gb1 += sum8(dot4(d[0], one, dot4(d[1], one, 0.0f)));
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int w = tid + e * kGradThreads;  // weight a * kIn + q
+            if (w < kH * kIn) {
+                const int a = w / kIn, q = w - a * kIn;
+                float acc = g1[e];
+                for (int t = 0; t < kTile; t += 4) {
+                    acc = dot4(*reinterpret_cast<const float4 *>(sQ + a * kRow + t),
+                               *reinterpret_cast<const float4 *>(sX + q * kRow + t), acc);
+                }
+                g1[e] = acc;
+            }
         }
     }
-    s = warp_sum(l);
-    if (lane == 0) atomicAdd(loss, s);
-    __syncthreads();
-    for (int q = threadIdx.x; q < kParams; q += blockDim.x) atomicAdd(&grad[q], G[q]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) atomicAdd(&grad[oW2 + (a0 + 16 * i) * kH + q0 + 16 * j], g2[i][j]);
+        const int w = tid + i * kGradThreads;
+        if (w < kH * kIn) atomicAdd(&grad[oW1 + w], g1[i]);
+    }
+    if (part == 0) {
+        atomicAdd(&grad[oB1 + row], gb1);
+        atomicAdd(&grad[oB2 + row], gb2);
+        atomicAdd(&grad[oW3 + row], gw3);
+    }
+    if (tid < kTile) {
+        gl = warp_sum(gl);
+        gb3 = warp_sum(gb3);
+        if ((tid & 31) == 0) {
+            atomicAdd(&grad[oB3], gb3);
+            atomicAdd(loss, gl);
+        }
+    }
 }
 
 // Adam (Kingma & Ba 2015) on the summed gradient times `scale`
@@ -550,8 +680,9 @@ int acfd_mlp_grad(const float *params, const float *X, const float *Y, int n, fl
         return ACFD_ERR_ARG;
     }
     if (n == 0) return ACFD_OK;
-    acfd::sensor::mlp_grad_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(params, X, Y, n, pos_weight,
-                                                                                     grad, loss);
+    const int tiles = (n - 1) / acfd::sensor::kTile + 1;
+    acfd::sensor::mlp_grad_kernel<<<std::min(tiles, acfd::sensor::kGradBlocks), acfd::sensor::kGradThreads, 0,
+                                    (cudaStream_t)stream>>>(params, X, Y, n, pos_weight, grad, loss);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ACFD_OK : acfd::cuda_status(e, "mlp_grad launch");
 }
