@@ -108,7 +108,7 @@ constexpr int kPlaneVariants = 6;
 constexpr int kPlaneWaves[kPlaneVariants] = {1, 2, 4, 1, 2, 4};
 constexpr bool kPlaneShare[kPlaneVariants] = {false, false, false, true, true, true};
 constexpr int kPlaneFirst = kTileVariants + kMarchVariants;
-constexpr long long kLineDefaultNodes = 1 << 18;  // computed nodes (acfd_init)
+constexpr long long kLineDefaultNodes = 1 << 17, kShareDefaultNodes = 1 << 19;  // computed nodes (acfd_init)
 constexpr int kStageVariants = kPlaneFirst + kPlaneVariants;
 static_assert(ACFD_BRICK_VARIANTS == kTileVariants && ACFD_STAGE_VARIANTS == kStageVariants &&
                   ACFD_PLANE_VARIANT == kPlaneFirst,
@@ -123,6 +123,27 @@ __global__ void set_scalar(double *p, double v)
 }  // namespace acfd
 
 using namespace acfd;
+
+// a ghost fill in one launch (launch_ghost_program): the copies in runs, the
+// other copies and the programs
+struct FillPlan {
+    int4 *tasks = nullptr;
+    int2 *single = nullptr;
+    int4 *progs = nullptr;
+    int ntask = 0, nsingle = 0, nprog = 0;
+    bool per_warp = false;       // a run is a warp's work, or a block's
+    std::vector<int4> h_tasks;   // host copies, for the fill of a batch
+    std::vector<int2> h_single;
+};
+
+// a run of a fill is a warp's work where the runs are short and more than a few,
+// otherwise a block's (copy_run)
+bool run_per_warp(const std::vector<int4> &tasks)
+{
+    long long copies = 0;
+    for (const int4 &t : tasks) copies += t.z;
+    return tasks.size() > 2 * 148 && copies < 512 * (long long)tasks.size();
+}
 
 // one piece of a profiled step (acfd_profile_step)
 struct StepPiece {
@@ -185,23 +206,20 @@ struct acfd_case {
     bool plain_kernels = false;    // use the global-memory stage kernels instead of the bricks
     bool bc_multi = false;         // one launch per ghost-fill phase instead of the fused launch
     unsigned *bcbar = nullptr;     // grid-barrier words of the fused ghost fill
-    int2 *bc_pairs = nullptr;      // ghost fill as one launch: copies (dst, src) -- base of the allocation
-    int bc_npairs = 0;
-    int4 *bc_progs = nullptr;      // ... and formula programs (dst, first op, op count)
-    int bc_nprog = 0;
-    int4 *bc_tasks = nullptr;      // the copies in runs (launch_ghost_program) ...
-    int bc_ntask = 0;
-    int2 *bc_single = nullptr;     // ... and the others
-    int bc_nsingle = 0;
-    int2 *bc_ops = nullptr;
+    // the ghost fill as one launch: bc[3] fills every ghost node, bc[s] those
+    // that a stage of sweep s reads (build_bc_program)
+    FillPlan bc[4];
+    int2 *bc_ops = nullptr;        // operations of the formula programs
+    char *bc_mem = nullptr, *xbc_mem = nullptr;  // device memory of the fills and operations
     GhostFaces bc_faces;
     bool bc_gather = false;        // the one-launch fill replaces the ordered launches
-    std::vector<int2> bc_copies;   // host copy of the copies of a copy-only fill
+    std::vector<int2> bc_copies;   // host copy of the copies (dst, src)
     // The X half steps as Y sweeps of the transposed state (build_xt): xg is
     // the grid with axes 0 and 1 exchanged, xU its three levels, xdid the
     // node types on it, xfl the sensor's x flags as the flags of its axis 1
     // ([2][xg.nn], slot 1), xmap the plane map of its Y sweep (box xbox), and
-    // the copy-only fill remapped to it (x_tasks, x_single).
+    // the copy-only fills remapped to it (xbc: for the next stage's sweep axis,
+    // or every ghost node).
     bool xt_ok = false;
     bool xt_all_forms = false;     // the transposed X sweep for the fast FP64 form too
     Grid xg = {};
@@ -210,10 +228,7 @@ struct acfd_case {
     uint8_t *xfl = nullptr;
     CUtensorMap xmap;
     int xbox[2] = {0, 0};
-    int4 *x_tasks = nullptr;
-    int x_ntask = 0;
-    int2 *x_single = nullptr;
-    int x_nsingle = 0;
+    FillPlan xbc[4];
     long long wait_limit = kWaitLimitDefault;  // polls of a plane-march wait (acfd_set_wait_limit)
     std::vector<StepPiece> *prof = nullptr;     // pieces of a step being profiled (acfd_profile_step)
     // ACFD_DEBUG=1: every stage and ghost fill is followed by a scan of its
@@ -465,6 +480,45 @@ struct GhostExprHash {
 
 }  // namespace
 
+// The four fills of a case (pairs[s], progs[s]) on the device, in one
+// allocation with the operations of their programs: the copies as tasks (runs,
+// no index loads) and single copies (ghost_tasks.h)
+bool make_fills(std::vector<int2> *const pairs[4], std::vector<int4> *const progs[4], const std::vector<int2> &ops,
+                FillPlan *f, int2 **d_ops, char **mem)
+{
+    std::vector<char> h;
+    auto put = [&](const void *p, size_t bytes) {
+        const size_t at = h.size();
+        h.resize(at + (bytes + 15) / 16 * 16);
+        if (bytes) memcpy(h.data() + at, p, bytes);
+        return at;
+    };
+    size_t at[4][3];
+    const size_t at_ops = put(ops.data(), ops.size() * sizeof(int2));
+    for (int s = 0; s < 4; ++s) {
+        ghost_copy_tasks(*pairs[s], f[s].h_tasks, f[s].h_single);
+        f[s].per_warp = run_per_warp(f[s].h_tasks);
+        f[s].ntask = (int)f[s].h_tasks.size();
+        f[s].nsingle = (int)f[s].h_single.size();
+        f[s].nprog = progs ? (int)progs[s]->size() : 0;
+        at[s][0] = put(f[s].h_tasks.data(), f[s].ntask * sizeof(int4));
+        at[s][1] = put(f[s].h_single.data(), f[s].nsingle * sizeof(int2));
+        at[s][2] = progs ? put(progs[s]->data(), f[s].nprog * sizeof(int4)) : 0;
+    }
+    if (cudaMalloc(mem, h.size() + 16) != cudaSuccess ||
+        cudaMemcpy(*mem, h.data(), h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (d_ops) *d_ops = reinterpret_cast<int2 *>(*mem + at_ops);
+    for (int s = 0; s < 4; ++s) {
+        f[s].tasks = reinterpret_cast<int4 *>(*mem + at[s][0]);
+        f[s].single = reinterpret_cast<int2 *>(*mem + at[s][1]);
+        f[s].progs = reinterpret_cast<int4 *>(*mem + at[s][2]);
+    }
+    return true;
+}
+
 bool build_bc_program(acfd_case *cs)
 {
     const acfd_partition_t &p = cs->part;
@@ -602,45 +656,29 @@ bool build_bc_program(acfd_case *cs)
         for (int s = 0; s < 3; ++s) cs->bc_faces.N[f][s] = p.N[f][s];
         for (int v = 0; v < 6; ++v) cs->bc_faces.given[f][v] = p.varBC[f][v];
     }
-    // the copies as tasks (runs, a block each, no index loads) and single
-    // copies (ghost_tasks.h)
-    std::vector<int4> tasks;
-    std::vector<int2> single;
-    ghost_copy_tasks(pairs, tasks, single);
-    auto al = [](size_t b) { return (b + 255) / 256 * 256; };
-    const size_t b_pairs = pairs.size() * sizeof(int2), b_progs = progs.size() * sizeof(int4);
-    const size_t b_ops = ops.size() * sizeof(int2), b_tasks = tasks.size() * sizeof(int4);
-    const size_t off_progs = al(b_pairs), off_ops = off_progs + al(b_progs), off_tasks = off_ops + al(b_ops);
-    const size_t off_single = off_tasks + al(b_tasks);
-    const size_t total = off_single + single.size() * sizeof(int2);
-    char *base = nullptr;
-    if (cudaMalloc(&base, total) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
+    // The fill of every ghost node, and for the stages inside a step the part of
+    // it that the next stage reads: no formula reads a node that the fill
+    // changes, so any part of it may be filled alone.
+    const int half = cs->model.sScheme == 1 ? 3 : 2;
+    std::vector<int2> part[3];
+    std::vector<int4> part_progs[3];
+    GhostReads reads(g.pitch, g.n[1], g.lo, g.hi, half, viscous(cs));
+    for (const int2 &q : pairs) {
+        const int r = reads(q.x);
+        for (int s = 0; s < 3; ++s) {
+            if (r >> s & 1) part[s].push_back(q);
+        }
     }
-    bool copied = cudaMemcpy(base, pairs.data(), b_pairs, cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemcpy(base + off_progs, progs.data(), b_progs, cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemcpy(base + off_ops, ops.data(), b_ops, cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemcpy(base + off_tasks, tasks.data(), b_tasks, cudaMemcpyHostToDevice) == cudaSuccess &&
-                  cudaMemcpy(base + off_single, single.data(), single.size() * sizeof(int2),
-                             cudaMemcpyHostToDevice) == cudaSuccess;
-    if (!copied) {
-        cudaGetLastError();
-        cudaFree(base);
-        return false;
+    for (const int4 &q : progs) {
+        const int r = reads(q.x);
+        for (int s = 0; s < 3; ++s) {
+            if (r >> s & 1) part_progs[s].push_back(q);
+        }
     }
-    cs->bc_pairs = reinterpret_cast<int2 *>(base);
-    cs->bc_npairs = (int)pairs.size();
-    cs->bc_progs = reinterpret_cast<int4 *>(base + off_progs);
-    cs->bc_nprog = (int)progs.size();
-    cs->bc_ops = reinterpret_cast<int2 *>(base + off_ops);
-    cs->bc_tasks = reinterpret_cast<int4 *>(base + off_tasks);
-    cs->bc_ntask = (int)tasks.size();
-    if (progs.empty()) {
-        cs->bc_copies = pairs;
-    }
-    cs->bc_single = reinterpret_cast<int2 *>(base + off_single);
-    cs->bc_nsingle = (int)single.size();
+    std::vector<int2> *const all_pairs[4] = {&part[0], &part[1], &part[2], &pairs};
+    std::vector<int4> *const all_progs[4] = {&part_progs[0], &part_progs[1], &part_progs[2], &progs};
+    if (!make_fills(all_pairs, all_progs, ops, cs->bc, &cs->bc_ops, &cs->bc_mem)) return false;
+    cs->bc_copies = std::move(pairs);
     return true;
 }
 
@@ -663,13 +701,11 @@ void release_xt(acfd_case *cs)
     cudaFree(cs->xU);
     cudaFree(cs->xdid);
     cudaFree(cs->xfl);
-    cudaFree(cs->x_tasks);
+    cudaFree(cs->xbc_mem);
+    cs->xbc_mem = nullptr;
     cs->xU = nullptr;
     cs->xdid = nullptr;
     cs->xfl = nullptr;
-    cs->x_tasks = nullptr;
-    cs->x_single = nullptr;
-    cs->x_ntask = cs->x_nsingle = 0;
     cs->xt_ok = false;
 }
 
@@ -677,7 +713,7 @@ void build_xt(acfd_case *cs)
 {
     const char *env = getenv("ACFD_X_TRANSPOSE");
     cs->xt_all_forms = env && strcmp(env, "all") == 0;
-    if ((env && env[0] == '0') || !cs->bc_gather || cs->bc_nprog != 0 || cs->bc_copies.empty() || !cs->pmaps_ok ||
+    if ((env && env[0] == '0') || !cs->bc_gather || cs->bc[3].nprog != 0 || cs->bc_copies.empty() || !cs->pmaps_ok ||
         cs->model.multidim != 0) {
         return;
     }
@@ -696,29 +732,27 @@ void build_xt(acfd_case *cs)
     if (xg.nn * 5 > (long long)INT32_MAX || (long long)g.n[2] * 5 > 65535) return;
     const PlaneTile pt = plane_tile(xg, 1, viscous(cs), 1, cs->sms);
     if (pt.BXp > 256 || pt.BC > 256) return;
-    // the copies on the transposed node indices, in destination order
-    const std::vector<int2> xc = transposed_copies_of(cs->bc_copies, g.pitch, g.n[0], g.n[1], xg.pitch);
-    std::vector<int4> tasks;
-    std::vector<int2> single;
-    ghost_copy_tasks(xc, tasks, single);
-    const size_t b_tasks = (tasks.size() * sizeof(int4) + 255) / 256 * 256;
-    char *prog = nullptr;
     if (cudaMalloc(&cs->xU, sizeof(double) * kLevels * kVars * (size_t)xg.nn) != cudaSuccess ||
         cudaMalloc(&cs->xdid, sizeof(int) * (size_t)xg.nn) != cudaSuccess ||
         cudaMalloc(&cs->xfl, 2 * (size_t)xg.nn) != cudaSuccess ||
-        cudaMemset(cs->xfl, 0, 2 * (size_t)xg.nn) != cudaSuccess ||
-        cudaMalloc(&prog, b_tasks + single.size() * sizeof(int2) + 16) != cudaSuccess ||
-        cudaMemcpy(prog, tasks.data(), tasks.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(prog + b_tasks, single.data(), single.size() * sizeof(int2), cudaMemcpyHostToDevice) !=
-            cudaSuccess) {
+        cudaMemset(cs->xfl, 0, 2 * (size_t)xg.nn) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(prog);
         return;  // the X sweep stays (acfd_finalize frees what was allocated)
     }
-    cs->x_tasks = reinterpret_cast<int4 *>(prog);
-    cs->x_ntask = (int)tasks.size();
-    cs->x_single = reinterpret_cast<int2 *>(prog + b_tasks);
-    cs->x_nsingle = (int)single.size();
+    // the copies on the transposed node indices, in destination order, and the
+    // parts that the sweeps read (axes 0 and 1 exchanged)
+    std::vector<int2> xc = transposed_copies_of(cs->bc_copies, g.pitch, g.n[0], g.n[1], xg.pitch);
+    const int half = cs->model.sScheme == 1 ? 3 : 2;
+    std::vector<int2> part[3];
+    GhostReads reads(xg.pitch, xg.n[1], xg.lo, xg.hi, half, viscous(cs));
+    for (const int2 &q : xc) {
+        const int r = reads(q.x);
+        if (r & 2) part[0].push_back(q);
+        if (r & 1) part[1].push_back(q);
+        if (r & 4) part[2].push_back(q);
+    }
+    std::vector<int2> *const all[4] = {&part[0], &part[1], &part[2], &xc};
+    if (!make_fills(all, nullptr, {}, cs->xbc, nullptr, &cs->xbc_mem)) return;
     PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
     if (!encode) return;
     const cuuint64_t dims[5] = {(cuuint64_t)xg.pitch, (cuuint64_t)xg.n[1], (cuuint64_t)xg.n[2], 5, 3};
@@ -740,17 +774,19 @@ void build_xt(acfd_case *cs)
 }
 
 int debug_scan(acfd_case *cs, int l, const char *what, int s);
-static int treat_boundary_fill(acfd_case *cs, int tn);
+static int treat_boundary_fill(acfd_case *cs, int tn, int next);
 
-int treat_boundary(acfd_case *cs, int tn)
+// next: the sweep axis of the stage that reads the level next (its ghost
+// nodes alone are filled), 3: every ghost node
+int treat_boundary(acfd_case *cs, int tn, int next = 3)
 {
-    const int st = treat_boundary_fill(cs, tn);
+    const int st = treat_boundary_fill(cs, tn, next);
     return st != ACFD_OK ? st : debug_scan(cs, tn, "ghost fill", -1);
 }
 
 // TreatBoundary (boundary_treatment.c:28-65): the bodies' ghost nodes, then
 // the domain's ghost shells
-static int treat_boundary_fill(acfd_case *cs, int tn)
+static int treat_boundary_fill(acfd_case *cs, int tn, int next)
 {
     if (cs->ib && ib_count(cs->ib) > 0) {
         cs->launches += ib_treat_launches(cs->ib, cs->part);
@@ -762,8 +798,9 @@ static int treat_boundary_fill(acfd_case *cs, int tn)
     double *U = level(cs, tn);
     if (cs->bc_gather) {
         ++cs->launches;
-        return launch_ghost_program(cs->grid, cs->mp, cs->bc_faces, cs->bc_tasks, cs->bc_ntask, cs->bc_single,
-                                    cs->bc_nsingle, cs->bc_progs, cs->bc_nprog, cs->bc_ops, U, cs->stream);
+        const FillPlan &f = cs->bc[next];
+        return launch_ghost_program(cs->grid, cs->mp, cs->bc_faces, f.tasks, f.ntask, f.per_warp, f.single, f.nsingle, f.progs,
+                                    f.nprog, cs->bc_ops, U, cs->stream);
     }
     if (!cs->bc_multi) {
         if (cs->bc_groups.empty()) {
@@ -954,7 +991,10 @@ const RkStage kRk3[3] = {{0.0, 1.0, ACFD_TO, ACFD_TO, ACFD_TN},
                          {3.0 / 4.0, 1.0 / 4.0, ACFD_TO, ACFD_TN, ACFD_TM},
                          {1.0 / 3.0, 2.0 / 3.0, ACFD_TO, ACFD_TM, ACFD_TO}};
 
-int discretize(acfd_case *cs, double dt_scale, int s)
+// next: the sweep axis of the half step after this one, when the level's other
+// ghost nodes are filled again before anything reads them (evolve); 3: every
+// fill is whole
+int discretize(acfd_case *cs, double dt_scale, int s, int next = 3)
 {
     const RkStage *rk = cs->model.tScheme == 0 ? kRk2 : kRk3;
     const int n = cs->model.tScheme == 0 ? 2 : 3;
@@ -964,7 +1004,7 @@ int discretize(acfd_case *cs, double dt_scale, int s)
             TRY(stage(cs, dt_scale, rk[q].coeA, rk[q].coeB, rk[q].to, rk[q].tn, rk[q].tm, s));
         }
         Piece p(cs, ACFD_PIECE_FILL, s, q);
-        TRY(treat_boundary(cs, rk[q].tm));
+        TRY(treat_boundary(cs, rk[q].tm, next == 3 ? 3 : q + 1 < n ? s : next));
     }
     return ACFD_OK;
 }
@@ -1039,16 +1079,16 @@ int stage_xt(acfd_case *cs, double dt_scale, double coeA, double coeB, int to, i
     return st;
 }
 
-int fill_xt(acfd_case *cs, int tn)
+int fill_xt(acfd_case *cs, int tn, int next)
 {
     ++cs->launches;
-    return launch_ghost_program(cs->xg, cs->mp, cs->bc_faces, cs->x_tasks, cs->x_ntask, cs->x_single,
-                                cs->x_nsingle, nullptr, 0, nullptr, cs->xU + (long long)tn * kVars * cs->xg.nn,
-                                cs->stream);
+    const FillPlan &f = cs->xbc[next];
+    return launch_ghost_program(cs->xg, cs->mp, cs->bc_faces, f.tasks, f.ntask, f.per_warp, f.single, f.nsingle,
+                                nullptr, 0, nullptr, cs->xU + (long long)tn * kVars * cs->xg.nn, cs->stream);
 }
 
 // DiscretizeTime along x on the transposed levels (the stages of discretize)
-int discretize_xt(acfd_case *cs, double dt_scale)
+int discretize_xt(acfd_case *cs, double dt_scale, int next)
 {
     const RkStage *rk = cs->model.tScheme == 0 ? kRk2 : kRk3;
     const int n = cs->model.tScheme == 0 ? 2 : 3;
@@ -1058,7 +1098,7 @@ int discretize_xt(acfd_case *cs, double dt_scale)
             TRY(stage_xt(cs, dt_scale, rk[q].coeA, rk[q].coeB, rk[q].to, rk[q].tn, rk[q].tm));
         }
         Piece p(cs, ACFD_PIECE_FILL, ACFD_X, q);
-        TRY(fill_xt(cs, rk[q].tm));
+        TRY(fill_xt(cs, rk[q].tm, next == 3 ? 3 : q + 1 < n ? ACFD_X : next));
     }
     return ACFD_OK;
 }
@@ -1101,15 +1141,22 @@ int evolve(acfd_case *cs)
     if (cs->model.multidim == 0) {
         const int c = cs->part.collapse;
         if (c >= 0 && c < 9) {
+            // Inside the step a fill writes the ghost nodes that the next stage
+            // reads (on 1023 x 511 x 5 nodes with a thin periodic z extent:
+            // 290 MB in the whole fill, 5-20 MB for an X or Y stage); the last
+            // half step fills all of them on the three levels, so that a
+            // finished step leaves what whole fills leave.
+            const bool parts = cs->bc_gather && !cs->debug && cs->model.sState == 0;
             for (int n = 0; n < 6 && kOrder[c][n] >= 0; ++n) {
                 const int ax = kOrder[c][n];
+                const int next = parts && n + 1 < 6 && kOrder[c][n + 1] >= 0 ? kOrder[c][n + 1] : 3;
                 if (ax == ACFD_X && xt) {
                     // a run of X half steps on the transposed state
                     if (n == 0 || kOrder[c][n - 1] != ACFD_X) TRY(xt_transpose(cs, true));
-                    TRY(discretize_xt(cs, 0.5));
+                    TRY(discretize_xt(cs, 0.5, next));
                     if (n + 1 >= 6 || kOrder[c][n + 1] != ACFD_X) TRY(xt_transpose(cs, false));
                 } else {
-                    TRY(discretize(cs, 0.5, ax));
+                    TRY(discretize(cs, 0.5, ax, next));
                 }
             }
         }
@@ -1374,7 +1421,8 @@ int acfd_last_error(char *buf, size_t len)
     return ACFD_OK;
 }
 
-int acfd_init(const acfd_partition_t *part, const acfd_model_t *model, acfd_case_t **out)
+// transposed: with the transposed levels of the X half steps where they apply
+static int init_case(const acfd_partition_t *part, const acfd_model_t *model, bool transposed, acfd_case_t **out)
 {
     if (!part || !model || !out) {
         set_error("acfd_init: null argument");
@@ -1409,12 +1457,15 @@ int acfd_init(const acfd_partition_t *part, const acfd_model_t *model, acfd_case
     }
     g.pitch = (part->n[0] + 7) & ~7;
     g.nn = (long long)g.pitch * g.n[1] * g.n[2];
-    // the FP64 form starts on the line march with equal shares where it is
-    // faster than the brick: step times on the brick and the line march, us:
-    // 33^3 nodes 211 / 566, 96x62x34 (WENO3) 310 / 373, 65^3 656 / 641,
-    // 158x96x60 1,558 / 1,356, 7.1 M nodes around bodies 11,415 / 8,675
-    if ((long long)(g.hi[0] - g.lo[0]) * (g.hi[1] - g.lo[1]) * (g.hi[2] - g.lo[2]) >= kLineDefaultNodes) {
-        for (int s = 0; s < 3; ++s) cs->tile_var[ACFD_FP64][s] = kPlaneFirst + 3;
+    // The FP64 form starts on the line march where it is faster than the brick,
+    // cut into segments below the nodes where equal shares are faster.  Step
+    // times on the brick, the segments and the shares, us: 33^3 nodes 228 / 255 /
+    // 576, 96x62x34 (WENO3) 297 / 284 / 354, 65^3 664 / 571 / 644, 89x69x49 631 /
+    // 589 / 650, 158x96x60 1,545 / 1,387 / 1,328, 7.1 M nodes around bodies 11,415
+    // / 14,616 / 8,675
+    const long long pin = (long long)(g.hi[0] - g.lo[0]) * (g.hi[1] - g.lo[1]) * (g.hi[2] - g.lo[2]);
+    if (pin >= kLineDefaultNodes) {
+        for (int s = 0; s < 3; ++s) cs->tile_var[ACFD_FP64][s] = kPlaneFirst + (pin >= kShareDefaultNodes ? 3 : 0);
     }
     ModelParams &m = cs->mp;
     m.gamma = model->gamma;
@@ -1493,7 +1544,7 @@ int acfd_init(const acfd_partition_t *part, const acfd_model_t *model, acfd_case
             return st;
         }
         cs->bc_gather = build_bc_program(cs);
-        build_xt(cs);
+        if (transposed) build_xt(cs);
     }
     if ((e = cudaStreamSynchronize(cs->stream)) != cudaSuccess) {
         st = cuda_status(e, "acfd_init");
@@ -1502,6 +1553,11 @@ int acfd_init(const acfd_partition_t *part, const acfd_model_t *model, acfd_case
     }
     *out = cs;
     return ACFD_OK;
+}
+
+int acfd_init(const acfd_partition_t *part, const acfd_model_t *model, acfd_case_t **out)
+{
+    return init_case(part, model, true, out);
 }
 
 int acfd_finalize(acfd_case_t *cs)
@@ -1521,7 +1577,7 @@ int acfd_finalize(acfd_case_t *cs)
     cudaFree(cs->cfl_out);
     cudaFree(cs->dstatus);
     cudaFree(cs->bcbar);
-    cudaFree(cs->bc_pairs);
+    cudaFree(cs->bc_mem);
     release_xt(cs);
     cudaFree(cs->dbg_word);
     cudaFree(cs->sensor_params);
@@ -2315,8 +2371,10 @@ struct acfd_batch {
     unsigned long long *d_counter = nullptr;  // work counters, one per stage launch of a step
     int *d_status = nullptr;
     BatchLevel *d_levels = nullptr;        // [ncase]
-    int4 *d_pairs = nullptr;               // ghost gather of the copy-only cases
+    int4 *d_pairs = nullptr;               // ghost copies of the copy-only cases (the persistent step's fill items)
     long long npairs = 0;
+    BatchFill fill[4];                     // ghost fill of the copy-only cases: every ghost node (3), or what a
+                                           // stage of sweep s reads
     std::vector<int> ordered_fill;         // cases whose ghosts need the ordered fill
     // plane-march stage kernels (all cases viscous or all inviscid, plane maps present)
     bool plane_ok = false, plane = false, visc = false;
@@ -2448,8 +2506,12 @@ int batch_step(acfd_batch *b)
             }
             ++launch;
             ++b->launches;
-            if (b->npairs > 0) {
-                TRY(launch_batch_gather(b->d_levels, b->d_pairs, b->npairs, sc.tm, b->stream));
+            // the ghost nodes that the next stage reads, all of them in the last
+            // half step (as in evolve)
+            const int next = h == 5 ? 3 : q + 1 < nstage ? s : order[h + 1];
+            const BatchFill &f = b->fill[next];
+            if (f.ntask + f.nsingle > 0) {
+                TRY(launch_batch_fill(b->d_levels, f, sc.tm, b->stream));
                 ++b->launches;
             }
             for (int c : b->ordered_fill) {
@@ -2457,7 +2519,7 @@ int batch_step(acfd_batch *b)
                 const cudaStream_t keep = cs->stream;
                 cs->stream = b->stream;
                 const long long l0 = cs->launches;
-                const int st = treat_boundary(cs, sc.tm);
+                const int st = treat_boundary(cs, sc.tm, cs->bc_gather && !cs->debug ? next : 3);
                 b->launches += cs->launches - l0;
                 cs->stream = keep;
                 TRY(st);
@@ -2509,13 +2571,10 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
     }
     for (int c = 0; c < ncase && st == ACFD_OK; ++c) {
         acfd_case *cs = nullptr;
-        st = acfd_init(&parts[c], &models[c], &cs);
-        if (st == ACFD_OK) {
-            // the batch kernels sweep x directly: a batch case holds no
-            // transposed levels
-            release_xt(cs);
-            b->cases.push_back(cs);
-        }
+        // the batch kernels sweep x directly: a batch case holds no transposed
+        // levels
+        st = init_case(&parts[c], &models[c], false, &cs);
+        if (st == ACFD_OK) b->cases.push_back(cs);
     }
     std::vector<BatchCase> hc(ncase);
     std::vector<CUtensorMap> hm((size_t)ncase * 3);
@@ -2524,6 +2583,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
     std::vector<const double *> vmax(ncase);
     std::vector<BatchLevel> lv(ncase);
     std::vector<int4> pairs;
+    std::vector<int4> ftasks[4], fsingle[4];  // the copies of the fills, the case in w (tasks) or x (single)
     for (int c = 0; c < ncase && st == ACFD_OK; ++c) {
         acfd_case *cs = b->cases[c];
         BatchCase &C = hc[c];
@@ -2551,14 +2611,16 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
         vmax[c] = cs->cfl_out;
         lv[c].U = cs->U;
         lv[c].nn = cs->grid.nn;
-        if (cs->bc_gather && cs->bc_nprog == 0) {
-            std::vector<int2> hp(cs->bc_npairs);
-            if ((e = cudaMemcpy(hp.data(), cs->bc_pairs, sizeof(int2) * hp.size(), cudaMemcpyDeviceToHost)) !=
-                cudaSuccess) {
-                st = cuda_status(e, "acfd_batch_init");
-            }
-            for (const int2 &q : hp) {
+        if (cs->bc_gather && cs->bc[3].nprog == 0) {
+            for (const int2 &q : cs->bc_copies) {
                 pairs.push_back(make_int4(c, q.x, q.y, 0));
+            }
+            for (int s = 0; s < 4; ++s) {
+                for (int4 t : cs->bc[s].h_tasks) {
+                    t.w = c;
+                    ftasks[s].push_back(t);
+                }
+                for (const int2 &q : cs->bc[s].h_single) fsingle[s].push_back(make_int4(c, q.x, q.y, 0));
             }
         } else {
             b->ordered_fill.push_back(c);
@@ -2654,6 +2716,23 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
             st = cuda_status(e, "acfd_batch_init");
         }
     }
+    for (int s = 0; s < 4 && st == ACFD_OK; ++s) {
+        BatchFill &f = b->fill[s];
+        f.ntask = (int)ftasks[s].size();
+        f.nsingle = (int)fsingle[s].size();
+        if (f.ntask + f.nsingle == 0) continue;
+        f.per_warp = run_per_warp(ftasks[s]);
+        if ((e = cudaMalloc(&f.tasks, sizeof(int4) * ((size_t)f.ntask + f.nsingle))) != cudaSuccess) {
+            st = cuda_status(e, "acfd_batch_init (ghost fill)");
+            break;
+        }
+        f.single = f.tasks + f.ntask;
+        if ((e = cudaMemcpy(f.tasks, ftasks[s].data(), sizeof(int4) * f.ntask, cudaMemcpyHostToDevice)) != cudaSuccess ||
+            (e = cudaMemcpy(f.single, fsingle[s].data(), sizeof(int4) * f.nsingle, cudaMemcpyHostToDevice)) !=
+                cudaSuccess) {
+            st = cuda_status(e, "acfd_batch_init (ghost fill)");
+        }
+    }
     // persistent step: plane maps for every case and copy-only ghost fills
     if (st == ACFD_OK && b->plane_ok && b->ordered_fill.empty()) {
         std::vector<long long> off((size_t)ncase + 1, 0);
@@ -2727,6 +2806,7 @@ int acfd_batch_finalize(acfd_batch_t *b)
     cudaFree(b->d_status);
     cudaFree(b->d_levels);
     cudaFree(b->d_pairs);
+    for (BatchFill &f : b->fill) cudaFree(f.tasks);
     cudaFree(b->d_planes);
     cudaFree(b->d_pmaps);
     cudaFree(b->d_pprefix);

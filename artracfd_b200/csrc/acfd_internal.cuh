@@ -87,8 +87,15 @@ struct BatchLevel {
     double *U;       // the case's state (3 levels x 5 variables x nn)
     long long nn;    // nodes per variable plane
 };
-// ghost fill of every case of a batch at level tn: pairs (case, dst, src, 0)
-int launch_batch_gather(const BatchLevel *cases, const int4 *pairs, long long count, int tn, cudaStream_t st);
+// ghost fill of the copy-only cases of a batch: runs of copies (first
+// destination, source offset, length, case), a warp or block each, and the other
+// copies (case, dst, src, 0)
+struct BatchFill {
+    int4 *tasks = nullptr, *single = nullptr;
+    int ntask = 0, nsingle = 0;
+    bool per_warp = true;
+};
+int launch_batch_fill(const BatchLevel *cases, const BatchFill &f, int tn, cudaStream_t st);
 // time step of every case from its CFL maximum (ComputeTimeStep, solve.c:152):
 // dt = cfl * min(d0/v0, min(d1/v1, d2/v2)) with vmax[c] the case's three maxima
 // and d the mesh sizes (3 per case)
@@ -399,9 +406,6 @@ struct FaceBox {
 };
 int launch_domain_boundary(const Grid &g, const ModelParams &m, const acfd_partition_t &part,
                            const FaceBox *boxes, int nbox, double *U, cudaStream_t st);
-// ghost fill as one gather: U[dst] = U[src] for every (dst, src) pair, all
-// five variables of the level U
-int launch_ghost_gather(const Grid &g, const int2 *pairs, int count, double *U, cudaStream_t st);
 // one level of the state (five variables, the x and y momenta exchanged),
 // an int array or a byte array transposed from grid gs to grid gd, whose axes
 // 0 and 1 are those of gs exchanged (every node, ghosts included)
@@ -424,11 +428,11 @@ constexpr int kGhostWall = 2;    // top := wall boundary node from the top (its 
 constexpr int kGhostImage = 3;   // (O, I) := image ghost of boundary point O and image node I
 constexpr int kGhostStack = 6;
 constexpr int kGhostMaxOps = 32;
-// tasks: runs of copies, a block each -- (first destination, source offset,
-// length <= 2048, 0); single: the other copies (dst, src); progs: (dst,
+// tasks: runs of copies, a warp (per_warp) or block each -- (first destination,
+// source offset, length <= kGhostLong, 0); single: the other copies (dst, src); progs: (dst,
 // first op, op count, 0); ops: (code | face << 3, node)
 int launch_ghost_program(const Grid &g, const ModelParams &m, const GhostFaces &F, const int4 *tasks, int ntask,
-                         const int2 *single, int nsingle, const int4 *progs, int nprog, const int2 *ops, double *U,
+                         bool per_warp, const int2 *single, int nsingle, const int4 *progs, int nprog, const int2 *ops, double *U,
                          cudaStream_t st);
 // all groups of one TreatBoundary in one cooperative launch with grid barriers;
 // bar: two device words (arrival count, generation), zero at first use

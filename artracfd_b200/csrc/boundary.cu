@@ -525,30 +525,52 @@ __device__ __forceinline__ void copy_node(double *U, long long nn, long long dst
     }
 }
 
-// Ghost fill of a case whose faces are all copies (periodic, outflow): every
-// changed node takes the value of one unchanged node, so the ordered faces
-// collapse into one gather (pairs: destination, source node index)
-__global__ void ghost_gather(long long nn, const int2 *__restrict__ pairs, int count, double *U)
+// A run of copies (first destination, source offset, length) by `threads`
+// threads, this one the t-th, up to four each in flight: their twenty loads
+// before their stores.  Rows of cubes (65 to 197 nodes) are a warp's work: a
+// block of 256 threads per row leaves half of them idle and keeps three rows in
+// flight on an SM (ten cases of 64^3 to 112^3: 45 us a fill, 37 with a warp per
+// row); rows of 1,029 nodes are a block's (a step of a 1024x512x4 grid 3.40 ms,
+// 3.44 with a warp per row), and so are the few rows of a small grid (a step of
+// 128x8x8 cells 140 us, 153 with a warp per row): run_per_warp.
+__device__ __forceinline__ void copy_run(double *U, long long nn, const int4 &c, int t, int threads)
 {
-    pdl_wait();
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
-        const int2 q = pairs[t];
-        copy_node(U, nn, q.x, q.y);
+    for (int q0 = t; q0 < c.z; q0 += 4 * threads) {
+        long long d[4];
+        double u[4][5];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int q = q0 + threads * r;
+            d[r] = q < c.z ? (long long)c.x + q : -1;
+            // a copy outside the level is dropped (the tasks cover exactly
+            // the fill's copies: tests/test_host.py)
+            if (d[r] >= nn || d[r] + c.y < 0 || d[r] + c.y >= nn) d[r] = -1;
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            if (d[r] >= 0) {
+#pragma unroll
+                for (int v = 0; v < 5; ++v) u[r][v] = U[v * nn + d[r] + c.y];
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            if (d[r] >= 0) {
+#pragma unroll
+                for (int v = 0; v < 5; ++v) U[v * nn + d[r]] = u[r][v];
+            }
+        }
     }
 }
 
-int launch_ghost_gather(const Grid &g, const int2 *pairs, int count, double *U, cudaStream_t st)
+// blocks of the runs of a fill: eight warps with a run each, or a run each
+__host__ __device__ inline int run_blocks(int ntask, bool per_warp)
 {
-    if (count <= 0) {
-        return ACFD_OK;
-    }
-    const int blocks = (int)blocks_for(count, 256);
-    cudaError_t e = launch_k(ghost_gather, dim3(blocks), dim3(256), 0, st, g.nn, pairs, count, U);
-    return e == cudaSuccess ? ACFD_OK : cuda_status(e, "ghost_gather launch");
+    return per_warp ? (ntask + 7) / 8 : ntask;
 }
 
 // Ghost fill as one launch of formulas (see build_bc_program): the first
-// nchunk blocks copy one run of nodes each; then a thread per remaining copy
+// blocks copy runs of nodes, a warp or a block each; then a thread per remaining copy
 // (U[dst] = U[src]) and a thread per postfix program -- LOAD pushes a node's
 // five values, INFLOW the given inflow state,
 // WALL replaces the top with the wall formula of a boundary node, IMAGE
@@ -556,45 +578,19 @@ int launch_ghost_gather(const Grid &g, const int2 *pairs, int count, double *U, 
 // ghost -- and store the result.  No node a program or pair reads is written
 // by the launch, so the threads need no ordering among themselves.
 __global__ void __launch_bounds__(256) ghost_program(long long nn, const int4 *__restrict__ tasks, int ntask,
-                                                     const int2 *__restrict__ single, int nsingle,
+                                                     bool per_warp, const int2 *__restrict__ single, int nsingle,
                                                      const int4 *__restrict__ progs, int nprog,
                                                      const int2 *__restrict__ ops, GhostFaces F, ModelParams mp,
                                                      double *U)
 {
     pdl_wait();
-    if ((int)blockIdx.x < ntask) {
-        // a run of copies, up to four per thread in flight: their twenty
-        // loads before their stores
-        const int4 c = tasks[blockIdx.x];
-        for (int q0 = threadIdx.x; q0 < c.z; q0 += 4 * blockDim.x) {
-            long long d[4];
-            double u[4][5];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                const int q = q0 + r * (int)blockDim.x;
-                d[r] = q < c.z ? (long long)c.x + q : -1;
-                // a copy outside the level is dropped (the tasks cover exactly
-                // the fill's copies: tests/test_host.py)
-                if (d[r] >= nn || d[r] + c.y < 0 || d[r] + c.y >= nn) d[r] = -1;
-            }
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                if (d[r] >= 0) {
-#pragma unroll
-                    for (int v = 0; v < 5; ++v) u[r][v] = U[v * nn + d[r] + c.y];
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                if (d[r] >= 0) {
-#pragma unroll
-                    for (int v = 0; v < 5; ++v) U[v * nn + d[r]] = u[r][v];
-                }
-            }
-        }
+    const int tb = run_blocks(ntask, per_warp);
+    if ((int)blockIdx.x < tb) {
+        const int q = per_warp ? (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5) : (int)blockIdx.x;
+        if (q < ntask) copy_run(U, nn, tasks[q], per_warp ? threadIdx.x & 31 : threadIdx.x, per_warp ? 32 : 256);
         return;
     }
-    const int t = ((int)blockIdx.x - ntask) * blockDim.x + threadIdx.x;
+    const int t = ((int)blockIdx.x - tb) * blockDim.x + threadIdx.x;
     if (t < nsingle) {
         const int2 q = single[t];
         copy_node(U, nn, q.x, q.y);
@@ -636,42 +632,55 @@ __global__ void __launch_bounds__(256) ghost_program(long long nn, const int4 *_
 }
 
 int launch_ghost_program(const Grid &g, const ModelParams &m, const GhostFaces &F, const int4 *tasks, int ntask,
-                         const int2 *single, int nsingle, const int4 *progs, int nprog, const int2 *ops, double *U,
+                         bool per_warp, const int2 *single, int nsingle, const int4 *progs, int nprog, const int2 *ops, double *U,
                          cudaStream_t st)
 {
     const long long rest = (long long)nsingle + nprog;
-    const long long blocks = ntask + (rest + 255) / 256;
+    const long long blocks = run_blocks(ntask, per_warp) + (rest + 255) / 256;
     if (blocks <= 0) {
         return ACFD_OK;
     }
-    cudaError_t e = launch_k(ghost_program, dim3((unsigned)blocks), dim3(256), 0, st, g.nn, tasks, ntask, single,
+    cudaError_t e = launch_k(ghost_program, dim3((unsigned)blocks), dim3(256), 0, st, g.nn, tasks, ntask, per_warp, single,
                              nsingle, progs, nprog, ops, F, m, U);
     return e == cudaSuccess ? ACFD_OK : cuda_status(e, "ghost_program launch");
 }
 
-// ghost fill of all cases of a batch in one launch (copy-only cases, see
-// ghost_gather)
-__global__ void batch_ghost_gather(const BatchLevel *__restrict__ cases, const int4 *__restrict__ pairs,
-                                   long long count, int tn)
+// ghost fill of all copy-only cases of a batch in one launch: a warp or block per run of
+// copies, then a thread per other copy (48 cases: one thread and one index load
+// per copy before)
+__global__ void __launch_bounds__(256) batch_ghost_fill(const BatchLevel *__restrict__ cases,
+                                                        const int4 *__restrict__ tasks, int ntask, bool per_warp,
+                                                        const int4 *__restrict__ single, int nsingle, int tn)
 {
     pdl_wait();
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < count;
-         t += (long long)gridDim.x * blockDim.x) {
-        const int4 q = pairs[t];
-        const BatchLevel c = cases[q.x];
-        copy_node(c.U + (long long)tn * 5 * c.nn, c.nn, q.y, q.z);
+    const int tb = run_blocks(ntask, per_warp);
+    if ((int)blockIdx.x < tb) {
+        const int q = per_warp ? (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5) : (int)blockIdx.x;
+        if (q >= ntask) return;
+        const int4 t = tasks[q];
+        const BatchLevel c = cases[t.w];
+        copy_run(c.U + (long long)tn * 5 * c.nn, c.nn, t, per_warp ? threadIdx.x & 31 : threadIdx.x,
+                 per_warp ? 32 : 256);
+        return;
     }
+    const int t = ((int)blockIdx.x - tb) * blockDim.x + threadIdx.x;
+    if (t >= nsingle) {
+        return;
+    }
+    const int4 q = single[t];
+    const BatchLevel c = cases[q.x];
+    copy_node(c.U + (long long)tn * 5 * c.nn, c.nn, q.y, q.z);
 }
 
-int launch_batch_gather(const BatchLevel *cases, const int4 *pairs, long long count, int tn, cudaStream_t st)
+int launch_batch_fill(const BatchLevel *cases, const BatchFill &f, int tn, cudaStream_t st)
 {
-    if (count <= 0) {
+    const int blocks = run_blocks(f.ntask, f.per_warp) + (f.nsingle + 255) / 256;
+    if (blocks <= 0) {
         return ACFD_OK;
     }
-    const long long want = (count + 255) / 256;
-    const unsigned blocks = (unsigned)(want < 148 * 64 ? want : 148 * 64);
-    cudaError_t e = launch_k(batch_ghost_gather, dim3(blocks), dim3(256), 0, st, cases, pairs, count, tn);
-    return e == cudaSuccess ? ACFD_OK : cuda_status(e, "batch_ghost_gather launch");
+    cudaError_t e = launch_k(batch_ghost_fill, dim3(blocks), dim3(256), 0, st, cases, (const int4 *)f.tasks, f.ntask,
+                             f.per_warp, (const int4 *)f.single, f.nsingle, tn);
+    return e == cudaSuccess ? ACFD_OK : cuda_status(e, "batch_ghost_fill launch");
 }
 
 // per-case dt of a batch, in the order of the reference's expression

@@ -4,12 +4,11 @@
 // The copies of a fill (destination, source node index) read only nodes the
 // fill does not change, so their order is free.  Runs of copies whose
 // destinations and sources both advance by one node (rows of a periodic or
-// outflow ghost plane) become tasks, one GPU block each, a run longer than
-// kGhostLong cut into pieces of at most that many (up to eight copies per
-// thread, four in flight).  A task is (first destination, source offset,
-// length, 0).  The copies of runs shorter than kGhostMinRun are returned one
-// by one (`single`, a thread each).  Rows of a ghost plane are not merged
-// into one task: on a 129^3 grid that made the fill slower.
+// outflow ghost plane) become tasks, one warp or block each (ghost_program), a
+// run longer than kGhostLong cut into pieces of at most that many.  A task is
+// (first destination, source offset, length, 0).  The
+// copies of runs shorter than kGhostMinRun are returned one by one (`single`, a
+// thread each).
 #pragma once
 
 #include <algorithm>
@@ -52,17 +51,77 @@ template <class Int2>
 std::vector<Int2> transposed_copies_of(const std::vector<Int2> &pairs, int pitch, int n0, int n1, int xpitch)
 {
     auto tr = [&](int q) {
-        const long long i = q % pitch, j = (q / pitch) % n1, k = q / ((long long)pitch * n1);
-        return (int)((k * n0 + i) * xpitch + j);
+        const unsigned row = (unsigned)q / (unsigned)pitch, k = row / (unsigned)n1;
+        const unsigned i = (unsigned)q - row * (unsigned)pitch, j = row - k * (unsigned)n1;
+        return (int)((k * (unsigned)n0 + i) * (unsigned)xpitch + j);
     };
+    // destination order by a table of the sources (a destination has one source)
+    int end = 0;
     std::vector<Int2> xc(pairs.size());
     for (size_t q = 0; q < xc.size(); ++q) {
         xc[q].x = tr(pairs[q].x);
         xc[q].y = tr(pairs[q].y);
+        end = std::max(end, xc[q].x + 1);
     }
-    std::sort(xc.begin(), xc.end(), [](const Int2 &a, const Int2 &b) { return a.x < b.x; });
+    std::vector<int> source((size_t)end, 0);  // source + 1, 0: no copy
+    for (const Int2 &c : xc) source[(size_t)c.x] = c.y + 1;
+    size_t n = 0;
+    for (int q = 0; q < end; ++q) {
+        if (source[(size_t)q] == 0) continue;
+        xc[n].x = q;
+        xc[n].y = source[(size_t)q] - 1;
+        ++n;
+    }
     return xc;
 }
+
+// The sweeps (bit s) whose stages read node q = (k * n1 + j) * pitch + i outside
+// the computed range [lo, hi): along s the stencil reaches `half` nodes beyond
+// it; a viscous flux also reads one node across, beside the nodes from the one
+// before the range to the one after it.
+struct GhostReads {
+    int pitch, n1;
+    int lo[3], hi[3];
+    int half;
+    bool viscous;
+    // the row of the node asked for last (nodes are asked for in order: one pair
+    // of divisions a row)
+    int first = 0, last = -1;
+    bool in[3], beside[3], near[3];
+
+    GhostReads(int pitch_, int n1_, const int *lo_, const int *hi_, int half_, bool viscous_)
+        : pitch(pitch_), n1(n1_), half(half_), viscous(viscous_)
+    {
+        for (int t = 0; t < 3; ++t) {
+            lo[t] = lo_[t];
+            hi[t] = hi_[t];
+        }
+    }
+    void set(int t, int c)
+    {
+        in[t] = c >= lo[t] && c < hi[t];
+        beside[t] = c == lo[t] - 1 || c == hi[t];
+        near[t] = c >= lo[t] - half && c < hi[t] + half;
+    }
+    int operator()(int q)
+    {
+        if (q < first || q > last) {
+            const int row = q / pitch, k = row / n1;
+            first = row * pitch;
+            last = first + pitch - 1;
+            set(1, row - k * n1);
+            set(2, k);
+        }
+        set(0, q - first);
+        int mask = 0;
+        for (int s = 0; s < 3; ++s) {
+            const int a = s == 0 ? 1 : 0, b = s == 2 ? 1 : 2;
+            const bool across = viscous && (in[s] || beside[s]) && ((beside[a] && in[b]) || (in[a] && beside[b]));
+            if ((near[s] && in[a] && in[b]) || across) mask |= 1 << s;
+        }
+        return mask;
+    }
+};
 
 #ifdef __CUDACC__
 inline void ghost_copy_tasks(const std::vector<int2> &pairs, std::vector<int4> &tasks, std::vector<int2> &single)

@@ -170,8 +170,8 @@ int acfd_synchronize(acfd_case_t *cs);
  * blocks, first with each tile's lines cut into equal segments, then with
  * equal shares of all tiles' planes per block.  The choice is kept per arithmetic form; the FP32 forms start on the
  * brick for X and the 4-wave plane march for Y and Z, the FP64 form on the
- * first brick below 262,144 computed nodes and on the plane march with one wave
- * of equal shares from there; acfd_autotune replaces these with the measured
+ * first brick below 131,072 computed nodes and on the plane march with one wave
+ * from there (segments; equal shares from 524,288 nodes); acfd_autotune replaces these with the measured
  * fastest. */
 #define ACFD_BRICK_VARIANTS 2
 #define ACFD_PLANE_VARIANT 5
