@@ -663,6 +663,7 @@ bool build_bc_program(acfd_case *cs)
     std::vector<int2> part[3];
     std::vector<int4> part_progs[3];
     GhostReads reads(g.pitch, g.n[1], g.lo, g.hi, half, viscous(cs));
+    for (auto &p : part) p.reserve(pairs.size());
     for (const int2 &q : pairs) {
         const int r = reads(q.x);
         for (int s = 0; s < 3; ++s) {
@@ -745,6 +746,7 @@ void build_xt(acfd_case *cs)
     const int half = cs->model.sScheme == 1 ? 3 : 2;
     std::vector<int2> part[3];
     GhostReads reads(xg.pitch, xg.n[1], xg.lo, xg.hi, half, viscous(cs));
+    for (auto &p : part) p.reserve(xc.size());
     for (const int2 &q : xc) {
         const int r = reads(q.x);
         if (r & 2) part[0].push_back(q);
@@ -2353,6 +2355,8 @@ int acfd_fhat_batch(const acfd_model_t *model, int s, int mode, const double *Us
 // all cases (ComputeTimeStep, EvolveFluidDynamics of every case, advanced
 // together; no reference counterpart for the batching itself)
 // ===========================================================================
+constexpr int kBatchWaves = 6;
+
 struct acfd_batch {
     std::vector<acfd_case *> cases;
     int mode = ACFD_FP32_BULK;
@@ -2635,6 +2639,15 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
     if (st == ACFD_OK) {
         b->visc = viscous(b->cases[0]);
         b->plane_ok = true;
+        // the lines of the cases are cut so that a launch has about kBatchWaves
+        // waves of blocks over all cases
+        long long tiles[3] = {0, 0, 0};
+        for (int c = 0; c < ncase; ++c) {
+            for (int s = 0; s < 3; ++s) {
+                const PlaneTile pt = plane_tile(b->cases[c]->grid, s, b->visc, 1, b->sms);
+                tiles[s] += (long long)pt.ntx * pt.ntc;
+            }
+        }
         for (int c = 0; c < ncase && b->plane_ok; ++c) {
             acfd_case *cs = b->cases[c];
             if (!cs->pmaps_ok || viscous(cs) != b->visc) {
@@ -2644,6 +2657,11 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
             for (int s = 0; s < 3; ++s) {
                 BatchPlane &P = hp[(size_t)c * 3 + s];
                 P.pt = plane_tile(cs->grid, s, b->visc, 1, b->sms);
+                const long long cuts = (kBatchWaves * 2LL * b->sms + tiles[s] - 1) / std::max(1LL, tiles[s]);
+                if (cuts < P.pt.nseg) {
+                    P.pt.nseg = (int)std::max(1LL, cuts);
+                    P.pt.nblk = P.pt.ntx * P.pt.ntc * P.pt.nseg;
+                }
                 P.gk = cs->grid;
                 const long long sy = (long long)cs->grid.pitch, sz = (long long)cs->grid.pitch * cs->grid.n[1];
                 if (s == 1) {

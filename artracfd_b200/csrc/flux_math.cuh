@@ -386,13 +386,12 @@ __device__ __forceinline__ T weno5(T f0, T f1, T f2, T f3, T f4)
 // the D^2.  75 operations a field in this form (102 with the candidates and
 // indicators written in the stencil values); the first differences also lose
 // less to cancellation (TGV 128^3, FP64 step 3.60 -> 3.38-3.43 ms, the shock
-// over a body 4.40 -> 4.16-4.20 ms).  The two normalisations share one reciprocal: the
-// product of the weight sums stays far inside the double range (it would
-// underflow in FP32, so this form is for FP64 only).
+// over a body 4.40 -> 4.16-4.20 ms).  FP64: the two normalisations share one
+// reciprocal (the product of the weight sums stays far inside the double range;
+// it would underflow in FP32, which takes two approximate reciprocals).
 template <typename T>
 __device__ __forceinline__ T weno5_departure(T e0, T e1, T e2, T e3, T e4, T lp, T ln)
 {
-    static_assert(sizeof(T) == sizeof(double), "FP64 form");
     const T eps = T(1.0e-6), c = T(13.0 / 12.0), h = T(0.5);
     const T D0 = e1 - e0, D1 = e2 - e1, D2 = e3 - e2, D3 = e4 - e3;
     const T t0 = c * D0 * D0, t1 = c * D1 * D1, t2 = c * D2 * D2, t3 = c * D3 * D3;
@@ -421,7 +420,11 @@ __device__ __forceinline__ T weno5_departure(T e0, T e1, T e2, T e3, T e4, T lp,
     const T Np = P12 * D0 + wp * D1 - P01 * X;
     const T Nn = M12 * D3 + wn * D2 + M01 * X;
     const T lp3 = lp * T(1.0 / 3.0), ln3 = ln * T(1.0 / 3.0);
-    return (lp3 * Np * Sn + ln3 * Nn * Sp) * rcp<T>(Sp * Sn);
+    if constexpr (sizeof(T) == sizeof(double)) {
+        return (lp3 * Np * Sn + ln3 * Nn * Sp) * rcp<T>(Sp * Sn);
+    } else {
+        return lp3 * Np * rcp<T>(Sp) + ln3 * Nn * rcp<T>(Sn);
+    }
 }
 
 // H+ + H- of one characteristic field from its six stencil values

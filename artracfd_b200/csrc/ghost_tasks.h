@@ -84,9 +84,9 @@ struct GhostReads {
     int lo[3], hi[3];
     int half;
     bool viscous;
-    // the row of the node asked for last (nodes are asked for in order: one pair
-    // of divisions a row)
-    int first = 0, last = -1;
+    // the row of the node asked for last and the answer inside the range along x
+    // (nodes are asked for in order: one pair of divisions a row)
+    int first = 0, last = -1, inside = 0;
     bool in[3], beside[3], near[3];
 
     GhostReads(int pitch_, int n1_, const int *lo_, const int *hi_, int half_, bool viscous_)
@@ -111,8 +111,14 @@ struct GhostReads {
             last = first + pitch - 1;
             set(1, row - k * n1);
             set(2, k);
+            inside = mask_at(lo[0]);
         }
-        set(0, q - first);
+        const int c = q - first;
+        return c >= lo[0] && c < hi[0] ? inside : mask_at(c);
+    }
+    int mask_at(int c)
+    {
+        set(0, c);
         int mask = 0;
         for (int s = 0; s < 3; ++s) {
             const int a = s == 0 ? 1 : 0, b = s == 2 ? 1 : 2;

@@ -106,7 +106,9 @@ __device__ __forceinline__ IfaceState<Real> march_state(const ModelParams &mp, c
 
 // characteristic split fluxes with WENO5 (NP = 6) or WENO3 (NP = 4) on every
 // field; W[m] holds node p-(NP/2-1)+m of interface p+1/2
-template <int S, int NP>
+// DIFF: WENO5 in first differences (weno5_pair), the two sides together: the
+// batch kernels of the FP32 forms (and every FP64 kernel)
+template <int S, int NP, bool DIFF>
 __device__ __forceinline__ void march_weno(const IfaceState<Real> &is, const Real (&W)[NP][5], Real G[5])
 {
     Real A[NP], Bv[NP];
@@ -132,7 +134,7 @@ __device__ __forceinline__ void march_weno(const IfaceState<Real> &is, const Rea
         }
         const Real lp = is.lp[r], ln = is.ln[r];
         Real hp, hn;
-        if constexpr (NP == 6 && sizeof(Real) == sizeof(double)) {
+        if constexpr (NP == 6 && (DIFF || sizeof(Real) == sizeof(double))) {
             hp = fast::weno5_pair<Real>(C, lp, ln);
             hn = Real(0);
         } else if constexpr (NP == 6) {
@@ -234,7 +236,7 @@ __device__ __forceinline__ void march_tdiff(const double *__restrict__ U, long l
 }
 
 // interface flux (convective minus viscous is added by the caller)
-template <int S, int NP, bool HYB>
+template <int S, int NP, bool HYB, bool DIFF = false>
 __device__ __forceinline__ void march_flux(const ModelParams &mp, const Real (&W)[NP][5], bool full, Real F[5])
 {
     constexpr int H = NP / 2;
@@ -242,12 +244,12 @@ __device__ __forceinline__ void march_flux(const ModelParams &mp, const Real (&W
     Real G[5];
     if constexpr (HYB && NP == 6) {
         if (full) {
-            march_weno<S, NP>(is, W, G);
+            march_weno<S, NP, DIFF>(is, W, G);
         } else {
             march_linear<S>(is, W, G);
         }
     } else {
-        march_weno<S, NP>(is, W, G);
+        march_weno<S, NP, DIFF>(is, W, G);
     }
     back_project<S>(is, G, F);
 }
@@ -264,7 +266,7 @@ __device__ __forceinline__ void march_flux(const ModelParams &mp, const Real (&W
 // The arithmetic of each evaluation is that of march_weno.  All 32 lanes of
 // the warp must call this together (plane-march kernels: every consumer lane
 // runs the same march).
-template <int S>
+template <int S, bool DIFF = false>
 __device__ __forceinline__ void march_flux_coop(const ModelParams &mp, const Real (&W)[6][5], bool full, Real F[5],
                                                 Real *wbuf)
 {
@@ -274,7 +276,7 @@ __device__ __forceinline__ void march_flux_coop(const ModelParams &mp, const Rea
     unsigned fm = __ballot_sync(kAll, full);
     if (__popc(fm) > 16) {
         if (full) {
-            march_weno<S, 6>(is, W, G);
+            march_weno<S, 6, DIFF>(is, W, G);
         } else {
             march_linear<S>(is, W, G);
         }
@@ -296,7 +298,7 @@ __device__ __forceinline__ void march_flux_coop(const ModelParams &mp, const Rea
                     A[m] = is.qk * W[m][0] - is.V[0] * W[m][1] - is.V[1] * W[m][2] - is.V[2] * W[m][3] + W[m][4];
                     Bv[m] = is.V[S] * W[m][0] - W[m][S + 1];
                 }
-                Real *o = wbuf + slot * 50;
+                Real *o = wbuf + slot * (DIFF ? 40 : 50);
 #pragma unroll
                 for (int r = 0; r < 5; ++r) {
                     Real C[6];
@@ -313,27 +315,45 @@ __device__ __forceinline__ void march_flux_coop(const ModelParams &mp, const Rea
                         }
                     }
                     const Real lp = is.lp[r], ln = is.ln[r];
+                    if constexpr (DIFF) {
 #pragma unroll
-                    for (int m = 0; m < 5; ++m) {
-                        o[(2 * r) * 5 + m] = lp * C[m];
-                        o[(2 * r + 1) * 5 + m] = ln * C[5 - m];
+                        for (int m = 0; m < 6; ++m) o[8 * r + m] = C[m];
+                        o[8 * r + 6] = lp;
+                        o[8 * r + 7] = ln;
+                    } else {
+#pragma unroll
+                        for (int m = 0; m < 5; ++m) {
+                            o[(2 * r) * 5 + m] = lp * C[m];
+                            o[(2 * r + 1) * 5 + m] = ln * C[5 - m];
+                        }
                     }
                 }
             }
             __syncwarp();
-            // task t = slot * 10 + 2 * field + side reads inputs [5t, 5t+5)
-            // and leaves its result in the first of them
-            const int ntask = __popc(chunk) * 10;
-            for (int t = lane; t < ntask; t += 32) {
-                Real *f = wbuf + t * 5;
-                f[0] = fast::weno5<Real>(f[0], f[1], f[2], f[3], f[4]);
+            if constexpr (DIFF) {
+                // task t = slot * 5 + field reads inputs [8t, 8t+8) and leaves
+                // its result in the first of them
+                const int ntask = __popc(chunk) * 5;
+                for (int t = lane; t < ntask; t += 32) {
+                    Real *f = wbuf + t * 8;
+                    const Real C[6] = {f[0], f[1], f[2], f[3], f[4], f[5]};
+                    f[0] = fast::weno5_pair<Real>(C, f[6], f[7]);
+                }
+            } else {
+                // task t = slot * 10 + 2 * field + side reads inputs [5t, 5t+5)
+                // and leaves its result in the first of them
+                const int ntask = __popc(chunk) * 10;
+                for (int t = lane; t < ntask; t += 32) {
+                    Real *f = wbuf + t * 5;
+                    f[0] = fast::weno5<Real>(f[0], f[1], f[2], f[3], f[4]);
+                }
             }
             __syncwarp();
             if (mine) {
-                const Real *o = wbuf + slot * 50;
+                const Real *o = wbuf + slot * (DIFF ? 40 : 50);
 #pragma unroll
                 for (int r = 0; r < 5; ++r) {
-                    G[r] = o[(2 * r) * 5] + o[(2 * r + 1) * 5];
+                    G[r] = DIFF ? o[8 * r] : o[(2 * r) * 5] + o[(2 * r + 1) * 5];
                 }
             }
             __syncwarp();

@@ -92,7 +92,7 @@ __device__ __forceinline__ void plane_share(const PlaneTile &pt, int Ls, long lo
 // (blk) so that the batched kernel runs the same code for a block of any case;
 // warps beyond the case's producer warp (a batch launch sized for its largest
 // tile) leave after the barrier set-up.
-template <int NP, bool VISC, bool HYB, bool SHARE = false>
+template <int NP, bool VISC, bool HYB, bool SHARE = false, bool DIFF = false>
 __device__ __forceinline__ void plane_yz_block(const Grid &g, const ModelParams &mp, const StageArgs &a,
                                                const PlaneTile &pt, const CUtensorMap *mapp, int blk,
                                                unsigned char *smem)
@@ -304,9 +304,9 @@ __device__ __forceinline__ void plane_yz_block(const Grid &g, const ModelParams 
             }
             Real F[5];
             if constexpr (HYB && NP == 6) {
-                march_flux_coop<S>(mp, W, full_w, F, coop + (size_t)warp * (kCoopBytes / sizeof(Real)));
+                march_flux_coop<S, DIFF>(mp, W, full_w, F, coop + (size_t)warp * (kCoopBytes / sizeof(Real)));
             } else {
-                march_flux<S, NP, HYB>(mp, W, full_w, F);
+                march_flux<S, NP, HYB, DIFF>(mp, W, full_w, F);
             }
             if (VISC) {
                 march_visc<S>(g, mp, Pc, Pn, Dc, Dn, F);
@@ -442,7 +442,7 @@ __device__ __forceinline__ bool consumers_barrier_or(bool abort, unsigned nbar)
     return any != 0u;
 }
 
-template <int NP, bool VISC, bool HYB, bool SHARE = false>
+template <int NP, bool VISC, bool HYB, bool SHARE = false, bool DIFF = false>
 __device__ __forceinline__ void plane_x_block(const Grid &g, const ModelParams &mp, const StageArgs &a,
                                               const PlaneTile &pt, const CUtensorMap *mapp, int blk,
                                               unsigned char *smem)
@@ -558,9 +558,9 @@ __device__ __forceinline__ void plane_x_block(const Grid &g, const ModelParams &
             }
             Real F[5];
             if constexpr (HYB && NP == 6) {
-                march_flux_coop<0>(mp, W, full_w, F, coop + (size_t)warp * (kCoopBytes / sizeof(Real)));
+                march_flux_coop<0, DIFF>(mp, W, full_w, F, coop + (size_t)warp * (kCoopBytes / sizeof(Real)));
             } else {
-                march_flux<0, NP, HYB>(mp, W, full_w, F);
+                march_flux<0, NP, HYB, DIFF>(mp, W, full_w, F);
             }
             if (VISC) {
                 Real Pc[4], Pn[4], Dc[2][2], Dn[2][2];
@@ -772,9 +772,9 @@ stage_plane_batch(const BatchCase *__restrict__ cases, const BatchPlane *__restr
     a.wait_limit = kWaitLimitDefault;
     const int blk = (int)(item - prefix[lo]);
     if (XS) {
-        plane_x_block<NP, VISC, HYB>(P.gk, C.mp, a, P.pt, pmaps + 3 * lo + s, blk, smem);
+        plane_x_block<NP, VISC, HYB, false, true>(P.gk, C.mp, a, P.pt, pmaps + 3 * lo + s, blk, smem);
     } else {
-        plane_yz_block<NP, VISC, HYB>(P.gk, C.mp, a, P.pt, pmaps + 3 * lo + s, blk, smem);
+        plane_yz_block<NP, VISC, HYB, false, true>(P.gk, C.mp, a, P.pt, pmaps + 3 * lo + s, blk, smem);
     }
 }
 
@@ -943,9 +943,9 @@ stage_plane_persistent(const BatchCase *__restrict__ cases, const BatchPlane *__
             a.flags = C.flags;
             a.wait_limit = kWaitLimitDefault;
             if constexpr (XS) {
-                plane_x_block<6, VISC, HYB>(P.gk, C.mp, a, P.pt, pmaps + 3 * c + s, s_blk, smem);
+                plane_x_block<6, VISC, HYB, false, true>(P.gk, C.mp, a, P.pt, pmaps + 3 * c + s, s_blk, smem);
             } else {
-                plane_yz_block<6, VISC, HYB>(P.gk, C.mp, a, P.pt, pmaps + 3 * c + s, s_blk, smem);
+                plane_yz_block<6, VISC, HYB, false, true>(P.gk, C.mp, a, P.pt, pmaps + 3 * c + s, s_blk, smem);
             }
             __syncthreads();
             if (threadIdx.x == 0) {
