@@ -442,12 +442,13 @@ int launch_domain_boundary_fused(const Grid &g, const ModelParams &m, const acfd
 
 // CFL wave-speed maximum, one launch: partials (kCflPartials doubles: four
 // per block, then a completion counter that must be zero when the buffer is
-// allocated) and out[4]: the three maxima and the count of blocks that met a
-// non-finite wave speed
+// allocated) and out: the three maxima, the count of blocks that met a
+// non-finite wave speed, and the case's error words where they are given (out[4]
+// from status, out[5] from ib_status)
 constexpr int kCflBlocks = 1184;  // 148 SMs x 8 blocks of 256 threads: enough warps to hide the loads
 constexpr int kCflPartials = 4 * kCflBlocks + 1;
 int launch_cfl(const Grid &g, const ModelParams &m, const double *U, const int *did,
-               double *partials, double *out, cudaStream_t st);
+               double *partials, double *out, const int *status, const int *ib_status, cudaStream_t st);
 
 // layout conversion between the reference node records and the device planes
 int launch_scatter_nodes(const Grid &g, const acfd_node_t *staged, double *U, int *flags,

@@ -275,8 +275,11 @@ __device__ __forceinline__ double vmax_of(double a, double b)
 // from 0 and a NaN never replaces a value (vmax_of), so no NaN enters and the
 // maximum does not depend on the order of combination.
 // div_x, div_y: division by the PIN extents along x and y (32-bit path).
+// status, ib_status (each optional): error words of the case, reported as
+// out[4] and out[5], so that one wait of the host brings everything; out may be
+// pinned host memory.
 __global__ void cfl_partial(Grid g, ModelParams mp, const double *U, const int *did, double *part, double *out,
-                            FastDiv div_x, FastDiv div_y)
+                            FastDiv div_x, FastDiv div_y, const int *status, const int *ib_status)
 {
     pdl_wait();
     const int Lx = g.hi[0] - g.lo[0], Ly = g.hi[1] - g.lo[1], Lz = g.hi[2] - g.lo[2];
@@ -401,6 +404,8 @@ __global__ void cfl_partial(Grid g, ModelParams mp, const double *U, const int *
         // out[3]: blocks that met a fluid node with a non-finite wave speed
         out[threadIdx.x] = v;
     }
+    if (threadIdx.x == 4 && status) out[4] = (double)__ldcg(status);
+    if (threadIdx.x == 5 && ib_status) out[5] = (double)__ldcg(ib_status);
     if (threadIdx.x == 0) {
         *count = 0u;  // for the next launch (stream order)
     }
@@ -832,12 +837,12 @@ int launch_domain_boundary_fused(const Grid &g, const ModelParams &m, const acfd
 }
 
 int launch_cfl(const Grid &g, const ModelParams &m, const double *U, const int *did, double *partials,
-               double *out, cudaStream_t st)
+               double *out, const int *status, const int *ib_status, cudaStream_t st)
 {
     const FastDiv div_x = make_fast_div((uint32_t)std::max(1, g.hi[0] - g.lo[0]));
     const FastDiv div_y = make_fast_div((uint32_t)std::max(1, g.hi[1] - g.lo[1]));
     cudaError_t e = launch_k(cfl_partial, dim3(kCflBlocks), dim3(256), 0, st, g, m, U, did, partials, out, div_x,
-                             div_y);
+                             div_y, status, ib_status);
     return e == cudaSuccess ? ACFD_OK : cuda_status(e, "cfl launch");
 }
 

@@ -1759,6 +1759,11 @@ int ib_fetch(IbState *ib, int n, double *v, double *Nf, double *Ne, double *Nv, 
     return ACFD_OK;
 }
 
+const int *ib_status_word(const IbState *ib)
+{
+    return ib && ib->count > 0 ? ib->status : nullptr;
+}
+
 int ib_check(IbState *ib, cudaStream_t st)
 {
     if (!ib || ib->count == 0) return ACFD_OK;
