@@ -212,6 +212,11 @@ struct acfd_case {
     FillPlan bc[4];
     int2 *bc_ops = nullptr;        // operations of the formula programs
     char *bc_mem = nullptr, *xbc_mem = nullptr;  // device memory of the fills and operations
+    // copies written by the stages themselves (FP64 form): StageArgs::push and
+    // push_list; push_state 0: not built, 1: ready, -1: the fill does not allow it
+    int *push = nullptr;           // [4][node], one table per reader; the records behind it
+    int4 *push_list = nullptr;
+    int push_state = 0;
     GhostFaces bc_faces;
     bool bc_gather = false;        // the one-launch fill replaces the ordered launches
     std::vector<int2> bc_copies;   // host copy of the copies (dst, src)
@@ -248,6 +253,11 @@ struct acfd_case {
 };
 
 namespace {
+
+long long pin_nodes(const Grid &g)
+{
+    return (long long)(g.hi[0] - g.lo[0]) * (g.hi[1] - g.lo[1]) * (g.hi[2] - g.lo[2]);
+}
 
 bool viscous(const acfd_case *cs)
 {
@@ -844,7 +854,9 @@ int debug_scan(acfd_case *cs, int l, const char *what, int s)
     return ACFD_OK;
 }
 
-int stage(acfd_case *cs, double dt_scale, double coeA, double coeB, int to, int tn, int tm, int p)
+// push: the sweep whose stage reads U[tm] next (3: whoever does); its ghost nodes
+// are written by this stage and no fill follows.  -1: a fill follows.
+int stage(acfd_case *cs, double dt_scale, double coeA, double coeB, int to, int tn, int tm, int p, int push = -1)
 {
     StageArgs a;
     a.Uo = level(cs, to);
@@ -864,6 +876,10 @@ int stage(acfd_case *cs, double dt_scale, double coeA, double coeB, int to, int 
     a.status = cs->dstatus;
     a.flags = cs->sensor_flags;
     a.wait_limit = cs->wait_limit;
+    if (push >= 0) {
+        a.push = cs->push + push * cs->grid.nn;
+        a.push_list = cs->push_list;
+    }
     for (int s = 0; s < 3; ++s) {
         const int v = cs->tile_var[cs->mode][s];
         a.var[s] = v < kTileVariants ? v : 0;
@@ -997,17 +1013,19 @@ const RkStage kRk3[3] = {{0.0, 1.0, ACFD_TO, ACFD_TO, ACFD_TN},
 // next: the sweep axis of the half step after this one, when the level's other
 // ghost nodes are filled again before anything reads them (evolve); 3: every
 // fill is whole
-int discretize(acfd_case *cs, double dt_scale, int s, int next = 3)
+int discretize(acfd_case *cs, double dt_scale, int s, int next = 3, bool push = false)
 {
     const RkStage *rk = cs->model.tScheme == 0 ? kRk2 : kRk3;
     const int n = cs->model.tScheme == 0 ? 2 : 3;
     for (int q = 0; q < n; ++q) {
+        const int reader = next == 3 ? 3 : q + 1 < n ? s : next;
         {
             Piece p(cs, ACFD_PIECE_STAGE, s, q);
-            TRY(stage(cs, dt_scale, rk[q].coeA, rk[q].coeB, rk[q].to, rk[q].tn, rk[q].tm, s));
+            TRY(stage(cs, dt_scale, rk[q].coeA, rk[q].coeB, rk[q].to, rk[q].tn, rk[q].tm, s, push ? reader : -1));
         }
+        if (push) continue;
         Piece p(cs, ACFD_PIECE_FILL, s, q);
-        TRY(treat_boundary(cs, rk[q].tm, next == 3 ? 3 : q + 1 < n ? s : next));
+        TRY(treat_boundary(cs, rk[q].tm, reader));
     }
     return ACFD_OK;
 }
@@ -1115,6 +1133,78 @@ int xt_transpose(acfd_case *cs, bool into)
                 : launch_transpose_state(cs->xU, cs->xg, level(cs, ACFD_TO), cs->grid, cs->stream);
 }
 
+// The ghost copies of every computed node, for stages that write them themselves
+// (StageArgs::push): a table for each reader of the level, those of a stage of
+// sweep s and (3) all.  Only for a fill of copies of computed nodes, and on the
+// small grids that run on the brick.  Called before a step is queued or captured.
+int ensure_push(acfd_case *cs)
+{
+    if (cs->push_state != 0 || cs->mode != ACFD_FP64) {
+        return ACFD_OK;
+    }
+    cs->push_state = -1;
+    const Grid &g = cs->grid;
+    if (!cs->bc_gather || cs->bc[3].nprog != 0 || cs->bc_copies.empty() || cs->model.multidim != 0 ||
+        pin_nodes(g) >= kLineDefaultNodes) {
+        return ACFD_OK;
+    }
+    const int half = cs->model.sScheme == 1 ? 3 : 2;
+    const int none = -1;
+    std::vector<int> place(4 * (size_t)g.nn, none), last((size_t)g.nn * 4, none);
+    std::vector<int4> list;
+    GhostReads reads(g.pitch, g.n[1], g.lo, g.hi, half, viscous(cs));
+    for (const int2 &q : cs->bc_copies) {
+        const int row = q.y / g.pitch, i = q.y - row * g.pitch, k = row / g.n[1], j = row - k * g.n[1];
+        if (i < g.lo[0] || i >= g.hi[0] || j < g.lo[1] || j >= g.hi[1] || k < g.lo[2] || k >= g.hi[2]) {
+            return ACFD_OK;  // the copy of a node that no stage owns
+        }
+        const int r = reads(q.x) | 8;
+        for (int s = 0; s < 4; ++s) {
+            if (!(r >> s & 1)) continue;
+            int &first = place[(size_t)s * g.nn + q.y], &at = last[(size_t)s * g.nn + q.y];
+            if (first < 0) {
+                first = at = (int)list.size();
+                list.push_back(make_int4(q.x, none, none, none));
+                continue;
+            }
+            int4 &c = list[(size_t)at];
+            if (c.y < 0) {
+                c.y = q.x;
+            } else if (c.z < 0) {
+                c.z = q.x;
+            } else if (c.w < 0) {
+                c.w = q.x;
+            } else {
+                // a full record: its last copy opens the next one
+                const int moved = c.w;
+                at = (int)list.size();
+                c.w = -at - 2;
+                list.push_back(make_int4(moved, q.x, none, none));
+            }
+        }
+    }
+    const size_t b_place = sizeof(int) * place.size(), b_list = sizeof(int4) * list.size();
+    if (cudaMalloc(&cs->push, (b_place + 15) / 16 * 16 + b_list) != cudaSuccess) {
+        cudaGetLastError();
+        return ACFD_OK;  // the fills stay
+    }
+    cs->push_list = reinterpret_cast<int4 *>(reinterpret_cast<char *>(cs->push) + (b_place + 15) / 16 * 16);
+    ACFD_CUDA(cudaMemcpyAsync(cs->push, place.data(), b_place, cudaMemcpyHostToDevice, cs->stream));
+    ACFD_CUDA(cudaMemcpyAsync(cs->push_list, list.data(), b_list, cudaMemcpyHostToDevice, cs->stream));
+    ACFD_CUDA(cudaStreamSynchronize(cs->stream));
+    cs->push_state = 1;
+    return ACFD_OK;
+}
+
+// whether the stages of sweep s write their ghost copies themselves: the FP64
+// form on the brick kernels, no bodies (their ghost values come before the
+// domain's), not while the pieces of a step are timed
+bool use_push(const acfd_case *cs, int s)
+{
+    return cs->mode == ACFD_FP64 && cs->push_state == 1 && cs->tile_var[ACFD_FP64][s] < kTileVariants &&
+           cs->maps_ok && !cs->plain_kernels && !cs->prof && !(cs->ib && ib_count(cs->ib) > 0);
+}
+
 // EvolveFluidDynamics (fluid_dynamics.c:55-116); the step dt is in d_dt
 int evolve(acfd_case *cs)
 {
@@ -1159,7 +1249,7 @@ int evolve(acfd_case *cs)
                     TRY(discretize_xt(cs, 0.5, next));
                     if (n + 1 >= 6 || kOrder[c][n + 1] != ACFD_X) TRY(xt_transpose(cs, false));
                 } else {
-                    TRY(discretize(cs, 0.5, ax, next));
+                    TRY(discretize(cs, 0.5, ax, next, parts && use_push(cs, ax)));
                 }
             }
         }
@@ -1466,7 +1556,7 @@ static int init_case(const acfd_partition_t *part, const acfd_model_t *model, bo
     // 576, 96x62x34 (WENO3) 297 / 284 / 354, 65^3 664 / 571 / 644, 89x69x49 631 /
     // 589 / 650, 158x96x60 1,545 / 1,387 / 1,328, 7.1 M nodes around bodies 11,415
     // / 14,616 / 8,675
-    const long long pin = (long long)(g.hi[0] - g.lo[0]) * (g.hi[1] - g.lo[1]) * (g.hi[2] - g.lo[2]);
+    const long long pin = pin_nodes(g);
     if (pin >= kLineDefaultNodes) {
         for (int s = 0; s < 3; ++s) cs->tile_var[ACFD_FP64][s] = kPlaneFirst + (pin >= kShareDefaultNodes ? 3 : 0);
     }
@@ -1581,6 +1671,7 @@ int acfd_finalize(acfd_case_t *cs)
     cudaFree(cs->dstatus);
     cudaFree(cs->bcbar);
     cudaFree(cs->bc_mem);
+    cudaFree(cs->push);
     release_xt(cs);
     cudaFree(cs->dbg_word);
     cudaFree(cs->sensor_params);
@@ -1644,6 +1735,7 @@ int acfd_sync_to_device(acfd_case_t *cs, const acfd_node_t *node, unsigned mask)
         return ACFD_ERR_ARG;
     }
     TRY(ensure_staging(cs));
+    TRY(ensure_push(cs));
     const size_t total = (size_t)cs->grid.n[0] * cs->grid.n[1] * cs->grid.n[2];
     TRY(upload_host(cs, cs->staging, node, total * sizeof(acfd_node_t)));
     TRY(launch_scatter_nodes(cs->grid, cs->staging, cs->U, cs->flags, mask, cs->stream));
@@ -1716,6 +1808,7 @@ int acfd_cfl(acfd_case_t *cs, double vmax[3])
 int acfd_evolve_fluid(acfd_case_t *cs, double dt)
 {
     TRY(check_case(cs));
+    TRY(ensure_push(cs));
     TRY(set_dt(cs, dt));
     TRY(evolve(cs));
     return ACFD_OK;
@@ -1758,6 +1851,7 @@ int acfd_evolve_fluid_graph(acfd_case_t *cs, double dt)
     if (cs->debug) {
         return acfd_evolve_fluid(cs, dt);  // the per-stage checks synchronize: no capture
     }
+    TRY(ensure_push(cs));
     TRY(set_dt(cs, dt));
     if (!cs->graph_exec || cs->graph_mode != cs->mode) {
         release_graph(cs);

@@ -55,6 +55,10 @@ struct StageArgs {
     int *status;          // device error word of the case
     const uint8_t *flags; // hybrid form: sensor flags [3][node] (1 = full WENO5)
     long long wait_limit; // polls of a plane-march wait for a TMA plane or a free ring slot
+    // FP64 brick, fills of copies only: the stage itself writes the ghost copies
+    // of the nodes it updates (push_copies); null: a fill follows the stage
+    const int *push = nullptr;       // [node] place of its copies in push_list, -1: none
+    const int4 *push_list = nullptr; // up to four destinations, -1: none; w < -1: three, and the next record -w-2
 };
 
 // polls of a bounded device wait before it gives up (kernels then write their
