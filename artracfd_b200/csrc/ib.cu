@@ -360,47 +360,6 @@ __device__ __forceinline__ void add_weighted(const double Uoh[6], double tiny, d
 // inverse distance weighting (immersed_boundary.c:413-473); type TYPED: fluid
 // nodes, TYPEF: fluid nodes that were fluid before this mapping (not joined),
 // r >= 1: nodes of body did in ghost layer r
-__device__ double idw(const IbGrid &G, const ModelParams &mp, const double *U, const int *flags,
-                      const unsigned char *joined, const int c[3], const double p[3], int h, int type, int did,
-                      double Uo[6], int *status)
-{
-    const Grid &g = G.g;
-    const long long nn = g.nn;
-    const int *fdid = flags;
-    const int *fgst = flags + 3 * nn;
-    double wsum = 0.0;
-    for (int n = 0; n < 6; ++n) Uo[n] = 0.0;
-    const int rmax = g.n[0] + g.n[1] + g.n[2];
-    for (int r = h, tally = 0; 0 == tally; ++r) {
-        if (r > rmax) {
-            atomicExch(status, 1);  // no qualifying node: the reference would not terminate
-            break;
-        }
-        for (int kh = -r; kh <= r; ++kh) {
-            for (int jh = -r; jh <= r; ++jh) {
-                for (int ih = -r; ih <= r; ++ih) {
-                    const int i = c[0] + ih, j = c[1] + jh, k = c[2] + kh;
-                    if (!in_pin(g, k, j, i)) continue;
-                    const long long id = node_of(g, i, j, k);
-                    if (did != fdid[id]) continue;
-                    if (type == kTypeF) {
-                        if (joined[id]) continue;
-                    } else if (type != kTypeD) {
-                        if (type != fgst[id]) continue;
-                    }
-                    ++tally;
-                    double ph[3], Uh[5], Uoh[6];
-                    node_point(G, k, j, i, ph);
-                    for (int v = 0; v < 5; ++v) Uh[v] = U[v * nn + id];
-                    to_primitive(mp.gamma, mp.gasR, Uh, Uoh);
-                    add_weighted(Uoh, G.tinyL, dist2(p, ph), wsum, Uo);
-                }
-            }
-        }
-    }
-    return wsum;
-}
-
 __device__ void orthogonal_space(const double N[3], double Ta[3], double Tb[3])
 {
     int mark = 2;
@@ -463,13 +422,20 @@ constexpr int kIdwBatch = 4;      // candidates per lane evaluated before the or
 
 // Inverse distance weighting by one warp (the candidates of the serial
 // version's k, j, i loop order, 32 x kIdwBatch at a time).  Every lane
-// evaluates candidates and writes w and Uoh[n] * w to the warp's shared
-// scratch; lanes 0..6 then add them in candidate order, each lane one sum
-// (Uo[0..5], wsum), so every sum takes exactly the serial version's
-// additions in the same order.  All lanes return the same values.
+// evaluates candidates; those that qualify write w and Uoh[n] * w to the warp's
+// shared scratch at their rank, one row per sum, and lanes 0..6 add their row in
+// that order (Uo[0..5], wsum), so every sum takes exactly the serial version's
+// additions in the same order.  All lanes return the same values.  The rows are
+// read ahead of the additions, whose chain (eight cycles a term) is then what a
+// sum costs: with the terms found one by one through the bits of the ballots,
+// and 64-bit divisions for the candidates' offsets, a layer of the ghost nodes
+// of eight spheres (5,200 nodes) took 17.1 us, 14.7 now.
+// joined (type kTypeF only): nodes left out.
+constexpr int kIdwRow = 32 * kIdwBatch + 5;  // doubles between the rows of the scratch (odd: no bank conflicts)
+
 __device__ double idw_warp(const IbGrid &G, const ModelParams &mp, const double *U, const int *flags,
-                           const int c[3], const double p[3], int h, int type, int did, double Uo[6],
-                           double (*sp)[8], int *status)
+                           const unsigned char *joined, const int c[3], const double p[3], int h, int type, int did,
+                           double Uo[6], double *sp, int *status)
 {
     const Grid &g = G.g;
     const long long nn = g.nn;
@@ -486,6 +452,7 @@ __device__ double idw_warp(const IbGrid &G, const ModelParams &mp, const double 
         }
         const long long side = 2 * r + 1;
         const long long total = side * side * side;
+        const bool small = total <= 0x7fffffffLL;  // 32-bit divisions
         for (long long base = 0; base < total; base += 32 * kIdwBatch) {
             bool qual[kIdwBatch];
             long long ids[kIdwBatch];
@@ -497,10 +464,19 @@ __device__ double idw_warp(const IbGrid &G, const ModelParams &mp, const double 
                 ids[b] = 0;
                 cc[b][0] = cc[b][1] = cc[b][2] = 0;
                 if (cand < total) {
-                    const int ih = (int)(cand % side) - r;
-                    const long long rest = cand / side;
-                    const int jh = (int)(rest % side) - r;
-                    const int kh = (int)(rest / side) - r;
+                    int ih, jh, kh;
+                    if (small) {
+                        const unsigned q = (unsigned)cand, w = (unsigned)side, row = q / w;
+                        ih = (int)(q - row * w) - r;
+                        kh = (int)(row / w);
+                        jh = (int)(row - (unsigned)kh * w) - r;
+                        kh -= r;
+                    } else {
+                        const long long row = cand / side;
+                        ih = (int)(cand % side) - r;
+                        jh = (int)(row % side) - r;
+                        kh = (int)(row / side) - r;
+                    }
                     const int i = c[0] + ih, j = c[1] + jh, k = c[2] + kh;
                     cc[b][0] = i;
                     cc[b][1] = j;
@@ -516,13 +492,18 @@ __device__ double idw_warp(const IbGrid &G, const ModelParams &mp, const double 
                 if (qual[b]) {
                     const long long id = ids[b];
                     bool ok = (did == fdid[id]);
-                    if (ok && type != kTypeD) ok = (type == fgst[id]);
+                    if (ok && type == kTypeF) {
+                        ok = !joined[id];
+                    } else if (ok && type != kTypeD) {
+                        ok = (type == fgst[id]);
+                    }
                     qual[b] = ok;
                 }
             }
-            unsigned mask[kIdwBatch];
+            int count = 0;
 #pragma unroll
             for (int b = 0; b < kIdwBatch; ++b) {
+                const unsigned mask = __ballot_sync(0xffffffffu, qual[b]);
                 if (qual[b]) {
                     const long long id = ids[b];
                     double ph[3], Uh[5], Uoh[6];
@@ -532,19 +513,18 @@ __device__ double idw_warp(const IbGrid &G, const ModelParams &mp, const double 
                     double w = dist2(p, ph);
                     if (G.tinyL > w) w = G.tinyL;
                     w = 1.0 / w;
-                    double *row = sp[32 * b + lane];
-                    for (int v = 0; v < 6; ++v) row[v] = Uoh[v] * w;
-                    row[6] = w;
+                    double *at = sp + count + __popc(mask & ((1u << lane) - 1u));
+                    for (int v = 0; v < 6; ++v) at[v * kIdwRow] = Uoh[v] * w;
+                    at[6 * kIdwRow] = w;
                 }
-                mask[b] = __ballot_sync(0xffffffffu, qual[b]);
-                tally += __popc(mask[b]);
+                count += __popc(mask);
             }
+            tally += count;
             __syncwarp();
             if (lane < 7) {
-#pragma unroll
-                for (int b = 0; b < kIdwBatch; ++b) {
-                    for (unsigned m = mask[b]; m; m &= m - 1) acc = acc + sp[32 * b + __ffs(m) - 1][lane];
-                }
+                const double *row = sp + lane * kIdwRow;
+#pragma unroll 8
+                for (int t = 0; t < count; ++t) acc = acc + row[t];
             }
             __syncwarp();
         }
@@ -562,9 +542,9 @@ __global__ void __launch_bounds__(kGhostWarps * 32) ib_ghost(IbGrid G, ModelPara
                                                              double *U, const int *flags, int tn, int r,
                                                              int *status)
 {
-    __shared__ double scratch[kGhostWarps][32 * kIdwBatch][8];
+    __shared__ double scratch[kGhostWarps][7 * kIdwRow];
     const int lane = threadIdx.x & 31;
-    double (*sp)[8] = scratch[threadIdx.x >> 5];
+    double *sp = scratch[threadIdx.x >> 5];
     const int count = min(nghost[r - 1], cap);  // an overflowing list has set the status
     ghosts += (long long)(r - 1) * cap;
     const Grid &g = G.g;
@@ -594,7 +574,7 @@ __global__ void __launch_bounds__(kGhostWarps * 32) ib_ghost(IbGrid G, ModelPara
                                map_node(pI[1], G.dmin[1], g.dd[1], G.ng[1]),
                                map_node(pI[2], G.dmin[2], g.dd[2], G.ng[2])};
             // ReconstructFlow (immersed_boundary.c:357-412)
-            double wsum = idw_warp(G, mp, Ut, flags, cI, pI, kIbR, kTypeD, 0, UoI, sp, status);
+            double wsum = idw_warp(G, mp, Ut, flags, nullptr, cI, pI, kIbR, kTypeD, 0, UoI, sp, status);
             const double w = 1.0 / wsum;
             const double rr[3] = {pO[0] - B.O[0], pO[1] - B.O[1], pO[2] - B.O[2]};
             double Vs[3];
@@ -629,7 +609,7 @@ __global__ void __launch_bounds__(kGhostWarps * 32) ib_ghost(IbGrid G, ModelPara
             UoG[5] = UoI[5];
         } else {
             const int cG[3] = {i, j, k};
-            const double ws = idw_warp(G, mp, Ut, flags, cG, pG, 1, r - 1, n + 1, UoG, sp, status);
+            const double ws = idw_warp(G, mp, Ut, flags, nullptr, cG, pG, 1, r - 1, n + 1, UoG, sp, status);
             for (int v = 0; v < 6; ++v) UoG[v] = UoG[v] / ws;
         }
         UoG[0] = UoG[4] / (UoG[5] * mp.gasR);
@@ -723,15 +703,18 @@ __global__ void sf_terms(IbGrid G, ModelParams mp, const DevBody *bodies, BoxLis
 }
 
 // Ordered sums and calibration of IntegrateSurfaceForce (solid_dynamics.c:
-// 139-168), one warp (block) per body: the warp walks the body's node box 128
+// 139-168), one warp (block) per body: the warp walks the body's node box 512
 // nodes at a time, stages the terms of the ghost nodes among them in shared
-// memory, and lanes 0..8 add Fp, Fv, Tt and lanes 9, 10 the pressure offset
-// sums of the variance test, each over the ghost nodes in box order.
-constexpr int kSumChunks = 4;
+// memory in box order, one row per term, and lanes 0..8 add Fp, Fv, Tt and lanes
+// 9, 10 the pressure offset sums of the variance test, each over the ghost nodes
+// in box order.  128 nodes at a time, with the terms found through the bits of
+// the ballots, eight spheres of 7 cells' radius took 114 us, 56 now.
+constexpr int kSumChunks = 16;
+constexpr int kSumRow = 32 * kSumChunks + 5;
 __global__ void __launch_bounds__(32) sf_sum(const DevBody *bodies, const long long *off, const double *terms,
                                              const unsigned char *valid, const int *lidN, double *force)
 {
-    __shared__ double rows[32 * kSumChunks][10];
+    __shared__ double rows[10 * kSumRow];
     const int lane = threadIdx.x;
     const int n = blockIdx.x;
     const DevBody &B = bodies[n];
@@ -740,33 +723,37 @@ __global__ void __launch_bounds__(32) sf_sum(const DevBody *bodies, const long l
     double acc = 0.0, p0 = 0.0;
     int gstN = 0;
     for (long long base = a; base < b; base += 32 * kSumChunks) {
-        unsigned mask[kSumChunks];
+        bool v[kSumChunks];
 #pragma unroll
         for (int c = 0; c < kSumChunks; ++c) {
             const long long t = base + 32 * c + lane;
-            const bool v = (t < b) && valid[t];
-            if (v) {
-#pragma unroll
-                for (int q = 0; q < 10; ++q) rows[32 * c + lane][q] = terms[10 * t + q];
-            }
-            mask[c] = __ballot_sync(0xffffffffu, v);
+            v[c] = (t < b) && valid[t];
         }
-        __syncwarp();
+        int count = 0;
 #pragma unroll
         for (int c = 0; c < kSumChunks; ++c) {
-            if (!mask[c]) continue;
-            if (0 == gstN) p0 = rows[32 * c + __ffs(mask[c]) - 1][9];
-            gstN += __popc(mask[c]);
+            const unsigned mask = __ballot_sync(0xffffffffu, v[c]);
+            if (v[c]) {
+                const long long t = base + 32 * c + lane;
+                double *at = rows + count + __popc(mask & ((1u << lane) - 1u));
+#pragma unroll
+                for (int q = 0; q < 10; ++q) at[q * kSumRow] = terms[10 * t + q];
+            }
+            count += __popc(mask);
+        }
+        __syncwarp();
+        if (count > 0) {
+            if (0 == gstN) p0 = rows[9 * kSumRow];
+            gstN += count;
             if (lane < 11) {
-                for (unsigned m = mask[c]; m; m &= m - 1) {
-                    const double *row = rows[32 * c + __ffs(m) - 1];
-                    if (lane < 9) {
-                        acc = acc + row[lane];
-                    } else if (lane == 9) {
-                        acc = acc + row[9] - p0;
-                    } else {
-                        acc = acc + (row[9] - p0) * (row[9] - p0);
-                    }
+                const double *row = rows + (lane < 9 ? lane : 9) * kSumRow;
+#pragma unroll 8
+                for (int t = 0; t < count; ++t) {
+                    const double x = row[t];
+                    const double y = lane == 10 ? (x - p0) * (x - p0) : x;
+                    acc = acc + y;
+                    const double less = acc - p0;
+                    acc = lane == 9 ? less : acc;
                 }
             }
         }
@@ -831,15 +818,31 @@ __global__ void col_scan(IbGrid G, const DevBody *bodies, BoxList bl, const int 
 // ---------------------------------------------------------------------------
 // node mapping
 // ---------------------------------------------------------------------------
-__global__ void map_init(Grid g, const DevBody *bodies, int *flags)
+// computed node t (x fastest); false beyond the last one.  32-bit divisions where
+// the count allows them (64-bit ones cost more than the loads of these kernels)
+__device__ __forceinline__ bool pin_node(const Grid &g, long long t, int &i, int &j, int &k)
 {
     const int Lx = g.hi[0] - g.lo[0], Ly = g.hi[1] - g.lo[1], Lz = g.hi[2] - g.lo[2];
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)Lx * Ly * Lz) return;
-    const int i = g.lo[0] + (int)(t % Lx);
-    const long long rest = t / Lx;
-    const int j = g.lo[1] + (int)(rest % Ly);
-    const int k = g.lo[2] + (int)(rest / Ly);
+    const long long total = (long long)Lx * Ly * Lz;
+    if (t >= total) return false;
+    if (total <= 0x7fffffffLL) {
+        const unsigned q = (unsigned)t, row = q / (unsigned)Lx, p = row / (unsigned)Ly;
+        i = g.lo[0] + (int)(q - row * (unsigned)Lx);
+        j = g.lo[1] + (int)(row - p * (unsigned)Ly);
+        k = g.lo[2] + (int)p;
+    } else {
+        const long long row = t / Lx;
+        i = g.lo[0] + (int)(t % Lx);
+        j = g.lo[1] + (int)(row % Ly);
+        k = g.lo[2] + (int)(row / Ly);
+    }
+    return true;
+}
+
+__global__ void map_init(Grid g, const DevBody *bodies, int *flags)
+{
+    int i, j, k;
+    if (!pin_node(g, (long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long nn = g.nn;
     const long long id = node_of(g, i, j, k);
     const int did = flags[id];
@@ -942,13 +945,8 @@ __device__ __forceinline__ int layer_of(const IbGrid &G, int q)
 __global__ void map_interface(IbGrid G, int *flags, unsigned char *joined)
 {
     const Grid &g = G.g;
-    const int Lx = g.hi[0] - g.lo[0], Ly = g.hi[1] - g.lo[1], Lz = g.hi[2] - g.lo[2];
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)Lx * Ly * Lz) return;
-    const int i = g.lo[0] + (int)(t % Lx);
-    const long long rest = t / Lx;
-    const int j = g.lo[1] + (int)(rest % Ly);
-    const int k = g.lo[2] + (int)(rest / Ly);
+    int i, j, k;
+    if (!pin_node(g, (long long)blockIdx.x * blockDim.x + threadIdx.x, i, j, k)) return;
     const long long nn = g.nn;
     const long long id = node_of(g, i, j, k);
     const int did = flags[id];
@@ -978,30 +976,48 @@ __global__ void map_interface(IbGrid G, int *flags, unsigned char *joined)
     flags[3 * nn + id] = gst;
 }
 
-// refill newly uncovered fluid nodes from fluid nodes that stayed fluid
-__global__ void map_refill(IbGrid G, ModelParams mp, double *U, int *flags, const unsigned char *joined, int *status)
+// refill newly uncovered fluid nodes from fluid nodes that stayed fluid: a thread
+// looks at a node, and the warp reconstructs the few that joined one after the
+// other (a thread per node searched its box alone: 105 us at 192^3 with eight
+// moving spheres, 48 now)
+constexpr int kRefillNodes = 8;
+__global__ void __launch_bounds__(kGhostWarps * 32) map_refill(IbGrid G, ModelParams mp, double *U, int *flags,
+                                                               const unsigned char *joined, int *status)
 {
+    __shared__ double scratch[kGhostWarps][7 * kIdwRow];
     const Grid &g = G.g;
-    const int Lx = g.hi[0] - g.lo[0], Ly = g.hi[1] - g.lo[1], Lz = g.hi[2] - g.lo[2];
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long)Lx * Ly * Lz) return;
-    const int i = g.lo[0] + (int)(t % Lx);
-    const long long rest = t / Lx;
-    const int j = g.lo[1] + (int)(rest % Ly);
-    const int k = g.lo[2] + (int)(rest / Ly);
+    const int lane = threadIdx.x & 31;
     const long long nn = g.nn;
-    const long long id = node_of(g, i, j, k);
-    if (!joined[id]) return;
-    const int c[3] = {i, j, k};
-    double p[3], Uo[6];
-    node_point(G, k, j, i, p);
-    const double ws = idw(G, mp, U, flags, joined, c, p, kIbR, kTypeF, 0, Uo, status);
-    for (int v = 0; v < 6; ++v) Uo[v] = Uo[v] / ws;
-    Uo[0] = Uo[4] / (Uo[5] * mp.gasR);
-    double Uc[5];
-    to_conservative(mp.gamma, Uo, Uc);
-    for (int v = 0; v < 5; ++v) U[v * nn + id] = Uc[v];
-    flags[nn + id] = -1;
+    // kRefillNodes nodes a thread, their marks loaded together (bit q of marks)
+    const long long first = (long long)blockIdx.x * kRefillNodes * blockDim.x + (threadIdx.x & ~31);
+    unsigned marks = 0;
+#pragma unroll
+    for (int q = 0; q < kRefillNodes; ++q) {
+        int i, j, k;
+        if (pin_node(g, first + (long long)q * blockDim.x + lane, i, j, k) && joined[node_of(g, i, j, k)]) {
+            marks |= 1u << q;
+        }
+    }
+#pragma unroll 1
+    for (int q = 0; q < kRefillNodes; ++q) {
+        for (unsigned m = __ballot_sync(0xffffffffu, marks >> q & 1u); m; m &= m - 1) {
+            int c[3];
+            pin_node(g, first + (long long)q * blockDim.x + __ffs(m) - 1, c[0], c[1], c[2]);
+            const long long id = node_of(g, c[0], c[1], c[2]);
+            double p[3], Uo[6];
+            node_point(G, c[2], c[1], c[0], p);
+            const double ws = idw_warp(G, mp, U, flags, joined, c, p, kIbR, kTypeF, 0, Uo, scratch[threadIdx.x >> 5],
+                                       status);
+            for (int v = 0; v < 6; ++v) Uo[v] = Uo[v] / ws;
+            Uo[0] = Uo[4] / (Uo[5] * mp.gasR);
+            double Uc[5];
+            to_conservative(mp.gamma, Uo, Uc);
+            if (lane == 0) {
+                for (int v = 0; v < 5; ++v) U[v * nn + id] = Uc[v];
+                flags[nn + id] = -1;
+            }
+        }
+    }
 }
 
 // facet table v0, e01, e02 (BuildTriangle, computational_geometry.c:449-462)
@@ -1809,7 +1825,7 @@ int ib_compute_geometric_field(IbState *ib, const Grid &g, const ModelParams &m,
     }
     map_interface<<<blocks_for(pin, 256), 256, 0, st>>>(G, flags, ib->joined);
     ACFD_CUDA(cudaGetLastError());
-    map_refill<<<blocks_for(pin, 128), 128, 0, st>>>(G, m, U, flags, ib->joined, ib->status);
+    map_refill<<<blocks_for(pin, kGhostWarps * 32 * kRefillNodes), kGhostWarps * 32, 0, st>>>(G, m, U, flags, ib->joined, ib->status);
     ACFD_CUDA(cudaGetLastError());
     if (part.gl >= 1) {
         const int rc = build_lists(ib, G, part, flags, st);
