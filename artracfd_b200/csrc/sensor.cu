@@ -633,7 +633,23 @@ int launch_sensor_flags(const Grid &g, const ModelParams &m, const double *U, co
     ACFD_CUDA(launch_k(sensor::rho_p_kernel, dim3((unsigned)((g.nn + 255) / 256)), dim3(256), 0, st, g.nn,
                        m.gamma - 1.0, U, rho_p));
     const long long groups = ((pin + 31) / 32) * 3;
-    const long long blocks = std::min<long long>((groups + sensor::kFlagWarps - 1) / sensor::kFlagWarps, 148LL * 8);
+    // as many blocks as are resident at once: a block loads the weights once and
+    // walks its groups (flags of 65^3 nodes 33 -> 27 us, of 129^3 145 -> 139 us, from eight
+    // blocks per SM of which three are resident)
+    static int resident[64] = {0};
+    int dev = 0;
+    ACFD_CUDA(cudaGetDevice(&dev));
+    int per_chip = dev >= 0 && dev < 64 ? resident[dev] : 0;
+    if (per_chip == 0) {
+        int per_sm = 0, sms = 0;
+        ACFD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sensor::flags_mma_kernel,
+                                                                sensor::kFlagWarps * 32, 0));
+        ACFD_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        per_chip = std::max(1, per_sm * sms);
+        if (dev >= 0 && dev < 64) resident[dev] = per_chip;
+    }
+    const long long blocks =
+        std::min<long long>((groups + sensor::kFlagWarps - 1) / sensor::kFlagWarps, per_chip);
     const FastDiv div_x = make_fast_div((uint32_t)(g.hi[0] - g.lo[0]));
     const FastDiv div_y = make_fast_div((uint32_t)(g.hi[1] - g.lo[1]));
     ACFD_CUDA(launch_k(sensor::flags_mma_kernel, dim3((unsigned)blocks), dim3(sensor::kFlagWarps * 32), 0, st, g,
