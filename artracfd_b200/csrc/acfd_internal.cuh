@@ -212,34 +212,42 @@ inline int plane_smem_bytes(const PlaneTile &pt, int s)
     return plane_smem_total(pt.BXp, pt.BC, s == 0 ? pt.TR * pt.NR : 0, pt.ncw);
 }
 
-// Line-march kernels of the FP64 form (sweep_line.cuh): one block per SM, eight
-// consumer warps (two per scheduler) and a producer's warpgroup.  The ring holds
-// planes of U[tn] and kLineOSlots tiles of U[to], each variable at a fixed
-// stride (one copy per variable), so that the kernel's shared-memory addresses
-// are immediate offsets.
-constexpr int kLineWarps = 8;
-constexpr int kLineThreads = (kLineWarps + 4) * 32;
-// launched with 384 x 168 registers: 256 x 232 + 128 x 40
-constexpr int kLineConsumerRegs = 232, kLineProducerRegs = 40;
-constexpr int kLinePlane = 368, kLineOPlane = 272;  // elements of a variable in a slot (128-byte multiples)
-constexpr int kLineOSlots = 4;
+// Line-march kernels of the FP64 form (sweep_line.cuh): one block per SM, consumer
+// warps and a producer's warpgroup, which gives its registers to them.  The ring
+// holds planes of U[tn] and tiles of U[to], each variable at a fixed stride (one
+// copy per variable), so that the kernel's shared-memory addresses are immediate
+// offsets.  Twelve consumer warps (three per scheduler) of 160 registers where a
+// thread fits into them, eight of 232 for the viscous Y and Z sweeps, which would
+// spill 200 bytes.  Stages on eight and on twelve warps, us: viscous X of 129^3
+// nodes 161 and 148; 1023x511x5 nodes inviscid X 155 and 143, Y 148 and 142, Z
+// 190 and 177; viscous Y and Z of 129^3 nodes 134 and 184.
+struct LineShape {
+    int warps, consumer_regs, producer_regs;  // registers: 512 x 128 or 384 x 168 at launch
+    int plane, oplane;                        // elements of a variable in a slot (128-byte multiples)
+    int oslots;                               // tiles of U[to]
+};
+__host__ __device__ constexpr LineShape line_shape(bool xs, bool visc)
+{
+    return (xs || !visc) ? LineShape{12, 160, 32, 512, 400, 3} : LineShape{8, 232, 40, 368, 272, 4};
+}
+__host__ __device__ constexpr int line_threads(const LineShape &c)
+{
+    return (c.warps + 4) * 32;
+}
 
 // slots of U[tn]: the planes of the stencil and those on their way (at most
-// np - 1 + kLineOSlots on Y and Z sweeps, 2 hv + kLineOSlots on X sweeps: see
-// the producers)
-__host__ __device__ constexpr int line_slots(int np)
+// np - 1 + oslots on Y and Z sweeps, 2 hv + oslots on X sweeps: see the producers)
+__host__ __device__ constexpr int line_slots(bool xs, int np, bool visc)
 {
-    return np - 1 + kLineOSlots;
+    return (xs ? (visc ? 2 : 0) : np - 1) + line_shape(xs, visc).oslots;
 }
-__host__ __device__ constexpr int line_x_slots(bool visc)
+__host__ __device__ constexpr int line_smem_bytes(bool xs, int np, bool visc)
 {
-    return (visc ? 2 : 0) + kLineOSlots;
+    return line_slots(xs, np, visc) * (5 * line_shape(xs, visc).plane * 8 + 2 * 8) +
+           line_shape(xs, visc).oslots * 5 * line_shape(xs, visc).oplane * 8;
 }
-__host__ __device__ constexpr int line_smem_bytes(int slots)
-{
-    return slots * (5 * kLinePlane * 8 + 2 * 8) + kLineOSlots * 5 * kLineOPlane * 8;
-}
-static_assert(line_smem_bytes(line_slots(6)) <= 227 * 1024, "shared memory of a block");
+static_assert(line_smem_bytes(false, 6, false) <= 227 * 1024 && line_smem_bytes(false, 6, true) <= 227 * 1024,
+              "shared memory of a block");
 
 struct LineTile {
     PlaneTile pt;
@@ -257,7 +265,8 @@ inline LineTile line_tile(const Grid &g, int s, bool visc, int waves, int sms, b
     const int T2 = (s == 2) ? 1 : 2, M = (s == 0) ? 1 : s;
     const int Lx = g.hi[0] - g.lo[0], Lt = g.hi[T2] - g.lo[T2], Ls = g.hi[M] - g.lo[M];
     const int hv = visc ? 1 : 0, hx = (s == 0) ? 3 : hv;
-    const int lines = (s == 0) ? kLineWarps * 30 + 2 : kLineWarps * 32, per_row = (s == 0) ? 2 : 0;
+    const LineShape shape = line_shape(s == 0, visc);
+    const int lines = (s == 0) ? shape.warps * 30 + 2 : shape.warps * 32, per_row = (s == 0) ? 2 : 0;
     double cost = -1.0;
     for (int ntx = 1; ntx <= (Lx > 0 ? Lx : 1); ++ntx) {
         LineTile lt = {};
@@ -270,12 +279,12 @@ inline LineTile line_tile(const Grid &g, int s, bool visc, int waves, int sms, b
         lt.OX = (pt.WX + 2) & ~1;
         if (pt.BXp > 256) continue;
         if (cost >= 0.0 && pt.WX < 12) break;
-        pt.NR = std::min(std::min(lines / pt.TR, Lt), std::min(kLinePlane / pt.BXp - 2 * hv, kLineOPlane / lt.OX));
+        pt.NR = std::min(std::min(lines / pt.TR, Lt), std::min(shape.plane / pt.BXp - 2 * hv, shape.oplane / lt.OX));
         if (pt.NR < 1) continue;
         pt.BC = pt.NR + 2 * hv;
         pt.ntc = (Lt + pt.NR - 1) / pt.NR;
-        pt.ncw = kLineWarps;
-        const double c = (double)pt.ntx * pt.ntc * (kLineWarps * 32 + 0.1 * pt.BXp * pt.BC);
+        pt.ncw = shape.warps;
+        const double c = (double)pt.ntx * pt.ntc * (shape.warps * 32 + 0.1 * pt.BXp * pt.BC);
         if (cost < 0.0 || c < cost) {
             best = lt;
             cost = c;

@@ -1,12 +1,12 @@
 // Line-march stage kernels of the fast FP64 form.
 //
-// One block per SM: eight consumer warps, two per scheduler with 232 registers
-// a thread, and a producer thread whose warpgroup gives its registers up.  The
-// producer streams the planes of U[tn] (the tile with the stencil's or the
-// viscous halo) and of U[to] (the tile alone) into rings of shared-memory
-// slots by TMA, one copy per variable, each variable at a fixed stride.  Y and
-// Z sweeps: a consumer thread walks one grid line along the sweep axis; X
-// sweeps march along y with a lane per node (stage_line_x).
+// One block per SM: eight or twelve consumer warps (line_shape) and a producer
+// thread whose warpgroup gives its registers up.  The producer streams the planes
+// of U[tn] (the tile with the stencil's or the viscous halo) and of U[to] (the
+// tile alone) into rings of shared-memory slots by TMA, one copy per variable,
+// each variable at a fixed stride.  Y and Z sweeps: a consumer thread walks one
+// grid line along the sweep axis; X sweeps march along y with a lane per node
+// (stage_line_x).
 //
 // What bounds it: the FP64 pipe and the issue slots beside it.  Measured on
 // B200: a scheduler issues an FP64 operation in two cycles (three for an FMA of
@@ -14,7 +14,7 @@
 // and every other instruction takes about 0.75 of a cycle more.  A viscous
 // WENO5 interface takes 651 FP64 and about 350 other instructions; at those
 // costs a stage of TGV 128^3 cannot take less than about 100 us, and it takes
-// 134 us on Y and Z and 161 us on X (187 and 198 us in the kernels before, 816
+// 134 us on Y and Z and 148 us on X (187 and 198 us in the kernels before, 816
 // FP64 instructions an interface and seven consumer warps on four schedulers;
 // DRAM 310 MB, 35% of the copy bandwidth).
 //  * WENO works on first differences (fast::weno5_departure).
@@ -28,11 +28,10 @@
 //    being held in registers: no window to shift, no spills.
 //  * U[to] arrives with the planes instead of by loads inside the march, and
 //    the node types are loaded a plane ahead.
-// Measured and left out: twelve consumer warps at 160 registers (viscous 184
-// us, spills; inviscid 142 against 151 us on a 1024x512x4 grid), the loop
-// unrolled twice (138 us), the next interface's state computed beside the
-// reconstruction (154 us), the acoustic field that runs downwind reconstructed
-// on one side only (143 us: 5% fewer FP64 operations, but longer chains).
+// Measured and left out, on eight warps at 134 us: the loop unrolled twice (138
+// us), the next interface's state computed beside the reconstruction (154 us), the
+// acoustic field that runs downwind reconstructed on one side only (143 us: 5%
+// fewer FP64 operations, but longer chains).
 //
 // The lines of a launch are cut as in the plane march (plane_next_item), by
 // one compiled kernel for both forms, so that the results do not depend on
@@ -314,7 +313,7 @@ __device__ __forceinline__ void viscous_part(const Gas &k, const Node &c, const 
 }  // namespace line
 
 template <int NP, bool VISC>
-__global__ void __launch_bounds__(kLineThreads, 1)
+__global__ void __launch_bounds__(line_threads(line_shape(false, VISC)), 1)
 stage_line(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_constant__ CUtensorMap map,
            const __grid_constant__ CUtensorMap omap)
 {
@@ -322,8 +321,9 @@ stage_line(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_consta
     constexpr int S = 1, T2 = 2;
     constexpr int H = NP / 2;
     constexpr int hv = VISC ? 1 : 0;
-    constexpr int NS = line_slots(NP), NO = kLineOSlots;
-    constexpr int PE = kLinePlane, OE = kLineOPlane;  // elements of a variable in a slot
+    constexpr LineShape shape = line_shape(false, VISC);
+    constexpr int NS = line_slots(false, NP, VISC), NO = shape.oslots;
+    constexpr int PE = shape.plane, OE = shape.oplane;  // elements of a variable in a slot
     constexpr unsigned kAll = 0xffffffffu;
     const PlaneTile &pt = lt.pt;
     double *ring = reinterpret_cast<double *>(smem);
@@ -334,7 +334,7 @@ stage_line(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_consta
     if (threadIdx.x == 0) {
         for (int q = 0; q < NS; ++q) {
             tma::mbar_init(full + q, 1);
-            tma::mbar_init(empty + q, kLineWarps);
+            tma::mbar_init(empty + q, shape.warps);
         }
     }
     __syncthreads();
@@ -365,16 +365,16 @@ stage_line(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_consta
     const int o2 = pt.swap ? 3 : 2, o3 = pt.swap ? 2 : 3;
     auto vg = [&](int v) { return v == 2 ? o2 : (v == 3 ? o3 : v); };
 
-    if (warp >= kLineWarps) {
+    if (warp >= shape.warps) {
         // the producer's warpgroup gives its registers to the consumers
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLineProducerRegs));
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(shape.producer_regs));
         // producer: plane q of the block's sequence into slot q % NS, its
         // variables in the kernel's order; with the plane of node p+H the
         // tile of U[to] of node p, which the same iteration updates.  A slot
         // is free again when the iteration that read it last is done, and by
         // then the tile of U[to] NO planes before this one is done with too
         // (NS <= 2 H - 1 + NO).
-        if (warp == kLineWarps && lane == 0) {
+        if (warp == shape.warps && lane == 0) {
             int q = 0, issued = 0, slot = 0, oslot = 0;
             unsigned phase = 1;  // parity of the empty barrier's phase before
             bool ok = true;
@@ -420,7 +420,7 @@ stage_line(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_consta
         return;
     }
 
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kLineConsumerRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(shape.consumer_regs));
     const line::Gas k = line::gas_of(mp, g, 0, S, T2);
     const long long nn = g.nn;
     const long long st = pt.st;  // node stride along the line
@@ -561,15 +561,16 @@ stage_line(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_consta
 // nodes a warp.
 // ---------------------------------------------------------------------------
 template <int NP, bool VISC>
-__global__ void __launch_bounds__(kLineThreads, 1)
+__global__ void __launch_bounds__(line_threads(line_shape(true, VISC)), 1)
 stage_line_x(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_constant__ CUtensorMap map,
              const __grid_constant__ CUtensorMap omap)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int H = NP / 2;
     constexpr int hv = VISC ? 1 : 0;
-    constexpr int NS = line_x_slots(VISC), NO = kLineOSlots;
-    constexpr int PE = kLinePlane, OE = kLineOPlane;
+    constexpr LineShape shape = line_shape(true, VISC);
+    constexpr int NS = line_slots(true, NP, VISC), NO = shape.oslots;
+    constexpr int PE = shape.plane, OE = shape.oplane;
     constexpr unsigned kAll = 0xffffffffu;
     const PlaneTile &pt = lt.pt;
     double *ring = reinterpret_cast<double *>(smem);
@@ -580,7 +581,7 @@ stage_line_x(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_cons
     if (threadIdx.x == 0) {
         for (int q = 0; q < NS; ++q) {
             tma::mbar_init(full + q, 1);
-            tma::mbar_init(empty + q, kLineWarps);
+            tma::mbar_init(empty + q, shape.warps);
         }
     }
     __syncthreads();
@@ -602,11 +603,11 @@ stage_line_x(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_cons
     // the kernel's frame: rho, y momentum, x momentum (the sweep's), z momentum, energy
     auto vg = [](int v) { return v == 1 ? 2 : (v == 2 ? 1 : v); };
 
-    if (warp >= kLineWarps) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kLineProducerRegs));
+    if (warp >= shape.warps) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(shape.producer_regs));
         // producer: with the plane of row j+hv the tile of U[to] of row j
         // (NS <= 2 hv + NO: see stage_line)
-        if (warp == kLineWarps && lane == 0) {
+        if (warp == shape.warps && lane == 0) {
             int q = 0, issued = 0, slot = 0, oslot = 0;
             unsigned phase = 1;
             bool ok = true;
@@ -649,7 +650,7 @@ stage_line_x(Grid g, ModelParams mp, StageArgs a, LineTile lt, const __grid_cons
         return;
     }
 
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kLineConsumerRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(shape.consumer_regs));
     const line::Gas k = line::gas_of(mp, g, 1, 0, 2);
     const long long nn = g.nn;
     const double rdt = (a.dt_scale * a.dt[0]) * g.dd[0];
@@ -777,7 +778,7 @@ static int launch_line_one(const Grid &g, const ModelParams &m, const StageArgs 
                            const CUtensorMap &map, const CUtensorMap &omap, cudaStream_t st)
 {
     static bool configured[64] = {false};
-    constexpr int smem = XS ? line_smem_bytes(line_x_slots(VISC)) : line_smem_bytes(line_slots(NP));
+    constexpr int smem = line_smem_bytes(XS, NP, VISC), threads = line_threads(line_shape(XS, VISC));
     auto kernel = XS ? stage_line_x<NP, VISC> : stage_line<NP, VISC>;
     int dev = 0;
     cudaGetDevice(&dev);
@@ -786,7 +787,7 @@ static int launch_line_one(const Grid &g, const ModelParams &m, const StageArgs 
         if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(stage_line)");
         if (dev >= 0 && dev < 64) configured[dev] = true;
     }
-    cudaError_t e = launch_k(kernel, dim3((unsigned)lt.pt.nblk), dim3(kLineThreads), smem, st, g, m, a, lt, map, omap);
+    cudaError_t e = launch_k(kernel, dim3((unsigned)lt.pt.nblk), dim3(threads), smem, st, g, m, a, lt, map, omap);
     return e == cudaSuccess ? ACFD_OK : cuda_status(e, "stage_line launch");
 }
 
