@@ -1,4 +1,5 @@
-// Plane-march stage kernels (fast FP64, FP32 and hybrid forms).
+// Plane-march stage kernels of the FP32 and hybrid forms (the FP64 form marches in
+// sweep_line.cuh, which shares the cutting of the lines, plane_next_item).
 //
 // Y and Z sweeps:
 // A block owns a tile of grid lines along the sweep axis s: WX consecutive x
@@ -19,7 +20,7 @@
 // persistent batch kernel may read a level that another SM rewrote since this
 // SM last cached it in L1.
 //
-// Included after sweep_march.cuh by sweep_fast.cu and sweep_fp32.cu.
+// Included after sweep_march.cuh by sweep_fp32.cu, and by sweep_line.cuh.
 #pragma once
 
 #include <utility>
@@ -235,27 +236,19 @@ __device__ __forceinline__ void plane_yz_block(const Grid &g, const ModelParams 
             }
         };
 
-        // A wait that gave up ends the block's march.  The FP64 form marks it
-        // and leaves at the end of the item, so that the march loop keeps a
-        // single exit (measured: FP64 stages 4% faster); the FP32 forms leave
-        // at once (measured: hybrid step 0.8% faster than with the mark).
-        constexpr bool kMarkFailure = sizeof(Real) == sizeof(double);
-        bool failed = false;
+        // a wait that gave up ends the block's march at once (with a mark read at
+        // the end of the item the hybrid step was 0.8% slower)
         Real W[NP][5];
     #pragma unroll
         for (int m = 0; m < NP - 1; ++m) {
-            if constexpr (kMarkFailure) {
-                if (!failed && !wait_plane(m)) failed = true;
-            } else {
-                if (!wait_plane(m)) return;
-            }
-            node_of_plane(plane(failed ? 0 : m), W[m]);
+            if (!wait_plane(m)) return;
+            node_of_plane(plane(m), W[m]);
         }
         Real Pc[4] = {Real(0), Real(0), Real(0), Real(0)};
         Real Dc[2][2] = {{Real(0), Real(0)}, {Real(0), Real(0)}};
         if (VISC) {
             march_prims(W[H - 1], cvinv, Pc);
-            tdiff(plane(failed ? 0 : H - 1), Dc);
+            tdiff(plane(H - 1), Dc);
         }
         for (int q = 0; q < H; ++q) {
             release(q);  // nodes p0-H .. p0-1 have no update
@@ -269,7 +262,7 @@ __device__ __forceinline__ void plane_yz_block(const Grid &g, const ModelParams 
             fl_ahead = fl[base + (long long)(p0 + 1) * st];
         }
         Real Fl[5];
-        for (int p = p0 - 1; p < p1 && !failed; ++p) {
+        for (int p = p0 - 1; p < p1; ++p) {
             const int qf = p - p0 + 2 * H;  // front node p+H
             const int q0 = p - p0 + H;      // node p
             const long long id = base + (long long)p * st;
@@ -288,14 +281,7 @@ __device__ __forceinline__ void plane_yz_block(const Grid &g, const ModelParams 
                 if (active) fl_ahead = fl[id + 3 * st];  // node p+3 <= p1+2, inside the march's planes
                 full_w = (fw != 0u);
             }
-            if (!wait_plane(qf)) {
-                if constexpr (kMarkFailure) {
-                    failed = true;
-                    break;
-                } else {
-                    return;
-                }
-            }
+            if (!wait_plane(qf)) return;
             node_of_plane(plane(qf), W[NP - 1]);
             Real Pn[4], Dn[2][2];
             if (VISC) {
@@ -349,17 +335,16 @@ __device__ __forceinline__ void plane_yz_block(const Grid &g, const ModelParams 
         if constexpr (SHARE) {
             // planes p1 .. p1+H-1 were read for the last time: free their slots
             // for the next item's planes
-            for (int q = NQ - H; q < NQ && !failed; ++q) {
+            for (int q = NQ - H; q < NQ; ++q) {
                 release(q);
             }
         }
-        if (failed) return;
         qbase += NQ;
     }
 }
 
 template <int NP, bool VISC, bool HYB, bool SHARE>
-__global__ void __launch_bounds__(kPlaneMaxThreads, sizeof(Real) == sizeof(float) ? 2 : 1)
+__global__ void __launch_bounds__(kPlaneMaxThreads, 2)
 stage_plane_yz(Grid g, ModelParams mp, StageArgs a, PlaneTile pt, const __grid_constant__ CUtensorMap map)
 {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -625,7 +610,7 @@ __device__ __forceinline__ void plane_x_block(const Grid &g, const ModelParams &
 
 
 template <int NP, bool VISC, bool HYB, bool SHARE>
-__global__ void __launch_bounds__(kPlaneMaxThreads, sizeof(Real) == sizeof(float) ? 2 : 1)
+__global__ void __launch_bounds__(kPlaneMaxThreads, 2)
 stage_plane_x(Grid g, ModelParams mp, StageArgs a, PlaneTile pt, const __grid_constant__ CUtensorMap map)
 {
     extern __shared__ __align__(128) unsigned char smem[];
