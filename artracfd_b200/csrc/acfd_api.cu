@@ -227,6 +227,7 @@ struct acfd_case {
     // the copy-only fills remapped to it (xbc: for the next stage's sweep axis,
     // or every ghost node).
     bool xt_ok = false;
+    bool xt_batch = false;         // the transposed levels belong to a batch's step alone
     bool xt_all_forms = false;     // the transposed X sweep for the fast FP64 form too
     Grid xg = {};
     double *xU = nullptr;
@@ -1039,7 +1040,7 @@ bool xt_eligible(const acfd_case *cs)
 {
     const bool form = cs->mode == ACFD_FP32_HYBRID || cs->mode == ACFD_FP32_BULK ||
                       (cs->xt_all_forms && cs->mode == ACFD_FP64 && cs->xline.ok);
-    return cs->xt_ok && !cs->debug && !cs->plain_kernels && form && !(cs->ib && ib_count(cs->ib) > 0);
+    return cs->xt_ok && !cs->xt_batch && !cs->debug && !cs->plain_kernels && form && !(cs->ib && ib_count(cs->ib) > 0);
 }
 
 // ... and do, when the X sweep's variant is a plane march (acfd_autotune
@@ -2485,6 +2486,19 @@ struct acfd_batch {
     long long *d_pprefix = nullptr;        // [3][ncase + 1] prefix sums of the plane blocks per sweep axis
     long long pblocks[3] = {0, 0, 0};
     int pthreads[3] = {0, 0, 0}, psmem[3] = {0, 0, 0};
+    // the X half steps as Y sweeps of the transposed states (build_batch_xt)
+    bool xt_ok = false;
+    BatchCase *d_xcases = nullptr;         // [ncase]
+    BatchPlane *d_xplanes = nullptr;       // [ncase][3], entry 1
+    CUtensorMap *d_xpmaps = nullptr;       // [ncase][3], entry 1
+    long long *d_xprefix = nullptr;        // [ncase + 1]
+    long long xblocks = 0;
+    int xthreads = 0, xsmem = 0;
+    BatchLevel *d_xlevels = nullptr;       // [ncase]
+    BatchFill xfill[4];
+    BatchTranspose *d_xtr = nullptr;       // [3][ncase]: U[TO] there, U[TO] back, the x flags there
+    long long *d_xtr_prefix = nullptr;     // [3][ncase + 1]
+    long long xtr_blocks[3] = {0, 0, 0};
     // persistent step (plane march, copy-only ghost fills): all stages of a
     // time step of every case in one launch (stage_plane_persistent)
     bool persist_ok = false, persist = false;
@@ -2498,6 +2512,7 @@ struct acfd_batch {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int graph_mode = -1;
+    bool graph_xt = false;
     long long graph_kernels = 0;
     long long launches = 0;
 };
@@ -2513,6 +2528,168 @@ void batch_release_graph(acfd_batch *b)
     b->exec = nullptr;
     b->graph = nullptr;
     b->graph_mode = -1;
+}
+
+// the copies of a fill of the whole batch to the device
+int upload_batch_fill(BatchFill &f, const std::vector<int4> &tasks, const std::vector<int4> &single)
+{
+    f.ntask = (int)tasks.size();
+    f.nsingle = (int)single.size();
+    if (f.ntask + f.nsingle == 0) return ACFD_OK;
+    f.per_warp = run_per_warp(tasks);
+    ACFD_CUDA(cudaMalloc(&f.tasks, sizeof(int4) * ((size_t)f.ntask + f.nsingle)));
+    f.single = f.tasks + f.ntask;
+    ACFD_CUDA(cudaMemcpy(f.tasks, tasks.data(), sizeof(int4) * f.ntask, cudaMemcpyHostToDevice));
+    ACFD_CUDA(cudaMemcpy(f.single, single.data(), sizeof(int4) * f.nsingle, cudaMemcpyHostToDevice));
+    return ACFD_OK;
+}
+
+// the lines of a batch's cases are cut so that a launch has about kBatchWaves waves
+// of blocks over all cases
+void batch_cuts(PlaneTile &pt, long long tiles, int sms)
+{
+    const long long cuts = (kBatchWaves * 2LL * sms + tiles - 1) / std::max(1LL, tiles);
+    if (cuts < pt.nseg) {
+        pt.nseg = (int)std::max(1LL, cuts);
+        pt.nblk = pt.ntx * pt.ntc * pt.nseg;
+    }
+}
+
+void release_batch_xt(acfd_batch *b)
+{
+    for (acfd_case *cs : b->cases) release_xt(cs);
+    void *mem[] = {b->d_xcases, b->d_xplanes, b->d_xpmaps, b->d_xprefix, b->d_xlevels, b->d_xtr, b->d_xtr_prefix};
+    for (void *p : mem) cudaFree(p);
+    for (BatchFill &f : b->xfill) {
+        cudaFree(f.tasks);
+        f.tasks = nullptr;
+    }
+    b->d_xcases = nullptr;
+    b->d_xplanes = nullptr;
+    b->d_xpmaps = nullptr;
+    b->d_xprefix = nullptr;
+    b->d_xlevels = nullptr;
+    b->d_xtr = nullptr;
+    b->d_xtr_prefix = nullptr;
+    b->xt_ok = false;
+}
+
+template <typename T>
+bool to_device(T *&p, const std::vector<T> &h)
+{
+    return cudaMalloc(&p, sizeof(T) * h.size()) == cudaSuccess &&
+           cudaMemcpy(p, h.data(), sizeof(T) * h.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+}
+
+// The X half steps of the plane-march launches as Y sweeps of the transposed
+// states, as in the single case (build_xt), when every case's fill is copies: the
+// X launch of ten viscous cases of 64..128 cells a side takes 597 us against 374
+// for Y, and their step 10.23 ms with the X launches, 9.29 ms with the transposes
+// (one launch over all cases each way).  The transposed levels double a case's state, so they are held only if
+// that leaves half of the free memory; without them the X sweep stays.
+void build_batch_xt(acfd_batch *b)
+{
+    const int ncase = (int)b->cases.size();
+    size_t need = 0, free_b = 0, total_b = 0;
+    for (const acfd_case *cs : b->cases) {
+        need += (sizeof(double) * kLevels * kVars + sizeof(int) + 2) * (size_t)((cs->grid.n[1] + 7) & ~7) *
+                cs->grid.n[0] * cs->grid.n[2];
+    }
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 2) {
+        cudaGetLastError();
+        return;
+    }
+    long long tiles = 0;
+    for (acfd_case *cs : b->cases) {
+        build_xt(cs);
+        cs->xt_batch = true;
+        if (!cs->xt_ok || cudaStreamSynchronize(cs->stream) != cudaSuccess) {
+            cudaGetLastError();
+            release_batch_xt(b);
+            return;
+        }
+        const PlaneTile pt = plane_tile(cs->xg, 1, b->visc, 1, b->sms);
+        tiles += (long long)pt.ntx * pt.ntc;
+    }
+    std::vector<BatchCase> xc(ncase);
+    std::vector<BatchPlane> xp((size_t)ncase * 3);
+    std::vector<CUtensorMap> xm((size_t)ncase * 3);
+    std::vector<long long> pre((size_t)ncase + 1, 0), tpre((size_t)3 * (ncase + 1), 0);
+    std::vector<BatchLevel> lv(ncase);
+    std::vector<BatchTranspose> tr((size_t)3 * ncase);
+    std::vector<int4> tasks[4], single[4];
+    bool ok = true;
+    for (int c = 0; c < ncase; ++c) {
+        const acfd_case *cs = b->cases[c];
+        const Grid &g = cs->grid, &xg = cs->xg;
+        xc[c].g = xg;
+        xc[c].mp = cs->mp;
+        xc[c].U = cs->xU;
+        xc[c].did = cs->xdid;
+        xc[c].flags = nullptr;
+        memset(xc[c].tiles, 0, sizeof(xc[c].tiles));
+        BatchPlane &P = xp[(size_t)c * 3 + 1];
+        P.pt = plane_tile(xg, 1, b->visc, 1, b->sms);
+        batch_cuts(P.pt, tiles, b->sms);
+        P.pt.swap = 0;
+        P.pt.st = (long long)xg.pitch;
+        P.pt.rs = (long long)xg.pitch * xg.n[1];
+        P.gk = xg;
+        ok = ok && P.pt.BXp == cs->xbox[0] && P.pt.BC == cs->xbox[1];
+        xm[(size_t)c * 3 + 1] = cs->xmap;
+        pre[(size_t)c + 1] = pre[c] + P.pt.nblk;
+        b->xthreads = std::max(b->xthreads, (P.pt.ncw + 1) * 32);
+        b->xsmem = std::max(b->xsmem, plane_smem_bytes(P.pt, 1));
+        lv[c].U = cs->xU;
+        lv[c].nn = xg.nn;
+        for (int s = 0; s < 4; ++s) {
+            for (int4 t : cs->xbc[s].h_tasks) {
+                t.w = c;
+                tasks[s].push_back(t);
+            }
+            for (const int2 &q : cs->xbc[s].h_single) single[s].push_back(make_int4(c, q.x, q.y, 0));
+        }
+        tr[c] = {cs->U, cs->xU, g.nn, xg.nn, g.pitch, xg.pitch, g.n[0], g.n[1]};
+        tr[(size_t)ncase + c] = {cs->xU, cs->U, xg.nn, g.nn, xg.pitch, g.pitch, xg.n[0], xg.n[1]};
+        tr[(size_t)2 * ncase + c] = {nullptr, cs->xfl + xg.nn, g.nn, xg.nn, g.pitch, xg.pitch, g.n[0], g.n[1]};
+        for (int q = 0; q < 3; ++q) {
+            long long *tp = tpre.data() + (size_t)q * (ncase + 1);
+            tp[c + 1] = tp[c] + transpose_tiles(q == 1 ? xg : g);
+        }
+    }
+    b->xblocks = pre[ncase];
+    for (int q = 0; q < 3; ++q) {
+        b->xtr_blocks[q] = tpre[(size_t)q * (ncase + 1) + ncase];
+        ok = ok && b->xtr_blocks[q] <= (long long)INT32_MAX;
+    }
+    ok = ok && to_device(b->d_xcases, xc) && to_device(b->d_xplanes, xp) && to_device(b->d_xpmaps, xm) &&
+         to_device(b->d_xprefix, pre) && to_device(b->d_xlevels, lv) && to_device(b->d_xtr, tr) &&
+         to_device(b->d_xtr_prefix, tpre);
+    for (int s = 0; s < 4; ++s) ok = ok && upload_batch_fill(b->xfill[s], tasks[s], single[s]) == ACFD_OK;
+    if (!ok) {
+        cudaGetLastError();
+        release_batch_xt(b);
+        return;
+    }
+    b->xt_ok = true;
+}
+
+// a case that was given bodies has left the transposed path (acfd_geo_upload)
+bool batch_use_xt(const acfd_batch *b)
+{
+    if (!b->xt_ok || !b->plane || b->persist) return false;
+    for (const acfd_case *cs : b->cases) {
+        if (!cs->xt_ok) return false;
+    }
+    return true;
+}
+
+int batch_transpose(acfd_batch *b, int which)
+{
+    const int ncase = (int)b->cases.size();
+    ++b->launches;
+    return launch_batch_transpose(b->d_xtr + (size_t)which * ncase, b->d_xtr_prefix + (size_t)which * (ncase + 1), ncase,
+                                  b->xtr_blocks[which], which != 2, b->stream);
 }
 
 // one time step of every case: CFL maxima, dt on the device, sensor flags
@@ -2535,6 +2712,8 @@ int batch_step(acfd_batch *b)
             b->launches += 2;
         }
     }
+    const bool xt = batch_use_xt(b);
+    if (xt && hybrid) TRY(batch_transpose(b, 2));
     static const int order[6] = {2, 1, 0, 0, 1, 2};
     struct Coef {
         double a, c;
@@ -2589,6 +2768,8 @@ int batch_step(acfd_batch *b)
     int launch = 0;
     for (int h = 0; h < 6; ++h) {
         const int s = order[h];
+        const bool hx = xt && s == 0;  // an X half step on the transposed states
+        if (hx && order[h - 1] != 0) TRY(batch_transpose(b, 0));
         for (int q = 0; q < nstage; ++q) {
             StageCoefs sc;
             sc.coeA = rk[q].a;
@@ -2597,7 +2778,11 @@ int batch_step(acfd_batch *b)
             sc.to = rk[q].to;
             sc.tn = rk[q].tn;
             sc.tm = rk[q].tm;
-            if (b->plane) {
+            if (hx) {
+                TRY(launch_stage_plane_batch(b->d_xcases, b->d_xplanes, b->d_xpmaps, b->d_xprefix, b->xblocks, ncase, sc,
+                                             b->d_dts, b->d_status, 1, b->visc, hybrid, b->xthreads, b->xsmem,
+                                             b->stream));
+            } else if (b->plane) {
                 TRY(launch_stage_plane_batch(b->d_cases, b->d_planes, b->d_pmaps, b->d_pprefix + (long long)s * (ncase + 1),
                                              b->pblocks[s], ncase, sc, b->d_dts, b->d_status, s, b->visc, hybrid,
                                              b->pthreads[s], b->psmem[s], b->stream));
@@ -2611,9 +2796,9 @@ int batch_step(acfd_batch *b)
             // the ghost nodes that the next stage reads, all of them in the last
             // half step (as in evolve)
             const int next = h == 5 ? 3 : q + 1 < nstage ? s : order[h + 1];
-            const BatchFill &f = b->fill[next];
+            const BatchFill &f = hx ? b->xfill[next] : b->fill[next];
             if (f.ntask + f.nsingle > 0) {
-                TRY(launch_batch_fill(b->d_levels, f, sc.tm, b->stream));
+                TRY(launch_batch_fill(hx ? b->d_xlevels : b->d_levels, f, sc.tm, b->stream));
                 ++b->launches;
             }
             for (int c : b->ordered_fill) {
@@ -2627,6 +2812,7 @@ int batch_step(acfd_batch *b)
                 TRY(st);
             }
         }
+        if (hx && order[h + 1] != 0) TRY(batch_transpose(b, 1));
     }
     return ACFD_OK;
 }
@@ -2673,8 +2859,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
     }
     for (int c = 0; c < ncase && st == ACFD_OK; ++c) {
         acfd_case *cs = nullptr;
-        // the batch kernels sweep x directly: a batch case holds no transposed
-        // levels
+        // its transposed levels, if any, come with the batch (build_batch_xt)
         st = init_case(&parts[c], &models[c], false, &cs);
         if (st == ACFD_OK) b->cases.push_back(cs);
     }
@@ -2737,8 +2922,6 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
     if (st == ACFD_OK) {
         b->visc = viscous(b->cases[0]);
         b->plane_ok = true;
-        // the lines of the cases are cut so that a launch has about kBatchWaves
-        // waves of blocks over all cases
         long long tiles[3] = {0, 0, 0};
         for (int c = 0; c < ncase; ++c) {
             for (int s = 0; s < 3; ++s) {
@@ -2755,11 +2938,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
             for (int s = 0; s < 3; ++s) {
                 BatchPlane &P = hp[(size_t)c * 3 + s];
                 P.pt = plane_tile(cs->grid, s, b->visc, 1, b->sms);
-                const long long cuts = (kBatchWaves * 2LL * b->sms + tiles[s] - 1) / std::max(1LL, tiles[s]);
-                if (cuts < P.pt.nseg) {
-                    P.pt.nseg = (int)std::max(1LL, cuts);
-                    P.pt.nblk = P.pt.ntx * P.pt.ntc * P.pt.nseg;
-                }
+                batch_cuts(P.pt, tiles[s], b->sms);
                 P.gk = cs->grid;
                 const long long sy = (long long)cs->grid.pitch, sz = (long long)cs->grid.pitch * cs->grid.n[1];
                 if (s == 1) {
@@ -2833,21 +3012,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
         }
     }
     for (int s = 0; s < 4 && st == ACFD_OK; ++s) {
-        BatchFill &f = b->fill[s];
-        f.ntask = (int)ftasks[s].size();
-        f.nsingle = (int)fsingle[s].size();
-        if (f.ntask + f.nsingle == 0) continue;
-        f.per_warp = run_per_warp(ftasks[s]);
-        if ((e = cudaMalloc(&f.tasks, sizeof(int4) * ((size_t)f.ntask + f.nsingle))) != cudaSuccess) {
-            st = cuda_status(e, "acfd_batch_init (ghost fill)");
-            break;
-        }
-        f.single = f.tasks + f.ntask;
-        if ((e = cudaMemcpy(f.tasks, ftasks[s].data(), sizeof(int4) * f.ntask, cudaMemcpyHostToDevice)) != cudaSuccess ||
-            (e = cudaMemcpy(f.single, fsingle[s].data(), sizeof(int4) * f.nsingle, cudaMemcpyHostToDevice)) !=
-                cudaSuccess) {
-            st = cuda_status(e, "acfd_batch_init (ghost fill)");
-        }
+        st = upload_batch_fill(b->fill[s], ftasks[s], fsingle[s]);
     }
     // persistent step: plane maps for every case and copy-only ghost fills
     if (st == ACFD_OK && b->plane_ok && b->ordered_fill.empty()) {
@@ -2883,7 +3048,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
             b->persist_blocks = bps * b->sms;
             b->persist_ok = true;
             // available (acfd_batch_set_kernel), not the default: measured
-            // 811 against 878 Mcell-steps/s for one launch per RK stage on the
+            // 859 against 911 Mcell-steps/s for one launch per RK stage on the
             // 48-case batch
             b->persist = false;
         } else {
@@ -2894,6 +3059,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
         acfd_batch_finalize(b);
         return st;
     }
+    if (b->plane_ok && b->ordered_fill.empty()) build_batch_xt(b);
     for (acfd_case *cs : b->cases) {
         cs->mode = ACFD_FP32_BULK;
     }
@@ -2908,6 +3074,7 @@ int acfd_batch_finalize(acfd_batch_t *b)
     }
     if (b->stream) cudaStreamSynchronize(b->stream);
     batch_release_graph(b);
+    release_batch_xt(b);
     for (acfd_case *cs : b->cases) {
         acfd_finalize(cs);
     }
@@ -2967,6 +3134,18 @@ int acfd_batch_set_precision(acfd_batch_t *b, int mode)
         hc[c].flags = (mode == ACFD_FP32_HYBRID) ? cs->sensor_flags : nullptr;
     }
     ACFD_CUDA(cudaMemcpy(b->d_cases, hc.data(), sizeof(BatchCase) * hc.size(), cudaMemcpyHostToDevice));
+    if (b->xt_ok) {
+        const size_t n = hc.size();
+        std::vector<BatchTranspose> tr(n);
+        ACFD_CUDA(cudaMemcpy(hc.data(), b->d_xcases, sizeof(BatchCase) * n, cudaMemcpyDeviceToHost));
+        ACFD_CUDA(cudaMemcpy(tr.data(), b->d_xtr + 2 * n, sizeof(BatchTranspose) * n, cudaMemcpyDeviceToHost));
+        for (size_t c = 0; c < n; ++c) {
+            hc[c].flags = (mode == ACFD_FP32_HYBRID) ? b->cases[c]->xfl : nullptr;
+            tr[c].src = b->cases[c]->sensor_flags;
+        }
+        ACFD_CUDA(cudaMemcpy(b->d_xcases, hc.data(), sizeof(BatchCase) * n, cudaMemcpyHostToDevice));
+        ACFD_CUDA(cudaMemcpy(b->d_xtr + 2 * n, tr.data(), sizeof(BatchTranspose) * n, cudaMemcpyHostToDevice));
+    }
     if (mode != b->mode) {
         batch_release_graph(b);
     }
@@ -2993,8 +3172,10 @@ int acfd_batch_advance(acfd_batch_t *b, const double *cfl, int steps, double *dt
         return ACFD_ERR_ARG;
     }
     ACFD_CUDA(cudaMemcpyAsync(b->d_cfl, cfl, sizeof(double) * ncase, cudaMemcpyHostToDevice, b->stream));
-    if (!b->exec || b->graph_mode != b->mode) {
+    const bool xt = batch_use_xt(b);
+    if (!b->exec || b->graph_mode != b->mode || b->graph_xt != xt) {
         batch_release_graph(b);
+        b->graph_xt = xt;
         ACFD_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
         const long long before = b->launches;
         int st = batch_step(b);

@@ -425,6 +425,20 @@ int launch_domain_boundary(const Grid &g, const ModelParams &m, const acfd_parti
 int launch_transpose_state(const double *src, const Grid &gs, double *dst, const Grid &gd, cudaStream_t st);
 int launch_transpose_int(const int *src, const Grid &gs, int *dst, const Grid &gd, cudaStream_t st);
 int launch_transpose_u8(const uint8_t *src, const Grid &gs, uint8_t *dst, const Grid &gd, cudaStream_t st);
+// the same for every case of a batch in one launch: block prefix[c] + t moves the
+// t-th 32 x 32 tile of case c (of the state's five variables, or of byte arrays)
+struct BatchTranspose {
+    const void *src;
+    void *dst;
+    long long src_nn, dst_nn;
+    int src_pitch, dst_pitch, na, nb;  // na x nb nodes a plane of the source
+};
+inline long long transpose_tiles(const Grid &gs)
+{
+    return (long long)((gs.n[0] + 31) / 32) * ((gs.n[1] + 31) / 32) * gs.n[2];
+}
+int launch_batch_transpose(const BatchTranspose *cases, const long long *prefix, int ncase, long long blocks, bool state,
+                           cudaStream_t st);
 // debug mode: add the count of non-finite values among U[0, count) to *word
 int launch_finite_scan(const double *U, long long count, int *word, cudaStream_t st);
 // ghost fill as one launch of formulas: per-face constants of the programs

@@ -855,14 +855,11 @@ int launch_cfl(const Grid &g, const ModelParams &m, const double *U, const int *
 // the tile of every variable, so that a thread has 4 * NV loads in flight
 // before the barrier (one variable per block leaves HBM half idle).
 template <typename T, int NV>
-__global__ void __launch_bounds__(256) transpose_xy(const T *__restrict__ src, long long src_nn, int src_pitch,
-                                                    T *__restrict__ dst, long long dst_nn, int dst_pitch, int na,
-                                                    int nb, bool swap_uv)
+__device__ __forceinline__ void transpose_tile(const T *__restrict__ src, long long src_nn, int src_pitch,
+                                               T *__restrict__ dst, long long dst_nn, int dst_pitch, int na, int nb,
+                                               bool swap_uv, int a0, int b0, int k)
 {
-    pdl_wait();
     __shared__ T tile[NV][32][33];
-    const int k = (int)blockIdx.z;
-    const int a0 = blockIdx.x * 32, b0 = blockIdx.y * 32;
     {
         const int a = a0 + threadIdx.x;
 #pragma unroll
@@ -885,6 +882,45 @@ __global__ void __launch_bounds__(256) transpose_xy(const T *__restrict__ src, l
             if (a < na && b < nb) dst[vd * dst_nn + ((long long)k * na + a) * dst_pitch + b] = tile[v][threadIdx.x][r];
         }
     }
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(256) transpose_xy(const T *__restrict__ src, long long src_nn, int src_pitch,
+                                                    T *__restrict__ dst, long long dst_nn, int dst_pitch, int na,
+                                                    int nb, bool swap_uv)
+{
+    pdl_wait();
+    transpose_tile<T, NV>(src, src_nn, src_pitch, dst, dst_nn, dst_pitch, na, nb, swap_uv, blockIdx.x * 32,
+                          blockIdx.y * 32, (int)blockIdx.z);
+}
+
+// the tiles of every case of a batch, one block each
+template <typename T, int NV>
+__global__ void __launch_bounds__(256) batch_transpose_xy(const BatchTranspose *__restrict__ cases,
+                                                          const long long *__restrict__ prefix, int ncase)
+{
+    pdl_wait();
+    int lo = 0, hi = ncase - 1;  // the case whose tiles contain this one
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (prefix[mid] <= (long long)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    const BatchTranspose C = cases[lo];
+    const unsigned t = (unsigned)((long long)blockIdx.x - prefix[lo]);
+    const unsigned ta = (C.na + 31) / 32, tb = (C.nb + 31) / 32;
+    transpose_tile<T, NV>((const T *)C.src, C.src_nn, C.src_pitch, (T *)C.dst, C.dst_nn, C.dst_pitch, C.na, C.nb,
+                          NV > 1, (int)(t % ta) * 32, (int)(t / ta % tb) * 32, (int)(t / (ta * tb)));
+}
+
+int launch_batch_transpose(const BatchTranspose *cases, const long long *prefix, int ncase, long long blocks, bool state,
+                           cudaStream_t st)
+{
+    if (blocks <= 0) return ACFD_OK;
+    cudaError_t e = state ? launch_k(batch_transpose_xy<double, 5>, dim3((unsigned)blocks), dim3(32, 8), 0, st, cases,
+                                     prefix, ncase)
+                          : launch_k(batch_transpose_xy<uint8_t, 1>, dim3((unsigned)blocks), dim3(32, 8), 0, st, cases,
+                                     prefix, ncase);
+    return e == cudaSuccess ? ACFD_OK : cuda_status(e, "batch transpose launch");
 }
 
 template <typename T, int NV>
