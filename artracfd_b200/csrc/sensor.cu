@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdint>
 
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
 #include "acfd_internal.cuh"
@@ -225,12 +226,17 @@ __device__ __forceinline__ float warp_sum(float v)
 // units 8 rg .. 8 rg + 7 of sample s forward and backward, then the weight
 // gradients -- sums over the samples -- are products of the stored rows, a
 // 2 x 2 patch of dW2 per thread, all in FP32.  The sums stay in registers over a
-// block's tiles and reach memory in one atomic per parameter and block.  What
-// bounds it is the latency of its six phases (16,384 samples: 256 blocks of one
-// tile); a warp reduction per weight and warp, with one thread per sample, took
-// 395 us for 16,384 samples.
+// block's tiles; a cluster of eight blocks adds its sums through distributed
+// shared memory and brings them to memory in one atomic per parameter.  (The
+// atomics of a parameter follow one another, and each rounds the running sum: one
+// per block, 256 of them for 16,384 samples, gave twice the error.)  What bounds
+// it is the latency of its six phases (16,384 samples: 256 blocks of one tile); a
+// warp reduction per weight and warp, with one thread per sample, took 395 us for
+// 16,384 samples.
+namespace cg = cooperative_groups;
 constexpr int kTile = 64, kRow = kTile + 4, kGradThreads = 256;
-constexpr int kGradBlocks = 2 * 148;
+constexpr int kGradBlocks = 2 * 148, kGradCluster = 8;
+static_assert(kGradBlocks % kGradCluster == 0 && kParams + 1 <= kGradCluster * kGradThreads, "grid of whole clusters");
 
 __device__ __forceinline__ float sum8(float v)
 {
@@ -245,10 +251,10 @@ __device__ __forceinline__ float dot4(float4 a, float4 b, float c)
     return fmaf(a.x, b.x, fmaf(a.y, b.y, fmaf(a.z, b.z, fmaf(a.w, b.w, c))));
 }
 
-__global__ void __launch_bounds__(kGradThreads) mlp_grad_kernel(const float *params, const float *X, const float *Y,
+__global__ void __cluster_dims__(kGradCluster, 1, 1) __launch_bounds__(kGradThreads) mlp_grad_kernel(const float *params, const float *X, const float *Y,
                                                                 int n, float pos_weight, float *grad, float *loss)
 {
-    __shared__ __align__(16) float P[(kParams + 3) / 4 * 4];
+    __shared__ __align__(16) float P[(kParams + 4) / 4 * 4];  // then the block's sums and its loss
     __shared__ __align__(16) float sX[kIn * kRow], sH1[kH * kRow], sD2[kH * kRow];
     __shared__ __align__(16) float sQ[kH * kRow];  // H2, then D1
     __shared__ __align__(16) float sdz[kTile];
@@ -354,15 +360,23 @@ __global__ void __launch_bounds__(kGradThreads) mlp_grad_kernel(const float *par
 #pragma unroll
         for (int r = 0; r < 8; ++r) sQ[(r0 + r) * kRow + s] = h1[r] > 0.0f ? d1[r] : 0.0f;
         // dW2 and the bias of layer 2 (D2 and H1 are complete)
+        float p2[2][2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};  // of 16 samples
         for (int t = 0; t < kTile; t += 4) {
             const float4 u0 = *reinterpret_cast<const float4 *>(sD2 + a0 * kRow + t);
             const float4 u1 = *reinterpret_cast<const float4 *>(sD2 + (a0 + 16) * kRow + t);
             const float4 v0 = *reinterpret_cast<const float4 *>(sH1 + q0 * kRow + t);
             const float4 v1 = *reinterpret_cast<const float4 *>(sH1 + (q0 + 16) * kRow + t);
-            g2[0][0] = dot4(u0, v0, g2[0][0]);
-            g2[0][1] = dot4(u0, v1, g2[0][1]);
-            g2[1][0] = dot4(u1, v0, g2[1][0]);
-            g2[1][1] = dot4(u1, v1, g2[1][1]);
+            p2[0][0] = dot4(u0, v0, p2[0][0]);
+            p2[0][1] = dot4(u0, v1, p2[0][1]);
+            p2[1][0] = dot4(u1, v0, p2[1][0]);
+            p2[1][1] = dot4(u1, v1, p2[1][1]);
+            if ((t & 12) == 12) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    g2[i >> 1][i & 1] += p2[i >> 1][i & 1];
+                    p2[i >> 1][i & 1] = 0.0f;
+                }
+            }
         }
         const float4 one = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
         {
@@ -380,35 +394,55 @@ __global__ void __launch_bounds__(kGradThreads) mlp_grad_kernel(const float *par
             const int w = tid + e * kGradThreads;  // weight a * kIn + q
             if (w < kH * kIn) {
                 const int a = w / kIn, q = w - a * kIn;
-                float acc = g1[e];
-                for (int t = 0; t < kTile; t += 4) {
-                    acc = dot4(*reinterpret_cast<const float4 *>(sQ + a * kRow + t),
-                               *reinterpret_cast<const float4 *>(sX + q * kRow + t), acc);
+                for (int t0 = 0; t0 < kTile; t0 += 16) {
+                    float acc = 0.0f;
+                    for (int t = t0; t < t0 + 16; t += 4) {
+                        acc = dot4(*reinterpret_cast<const float4 *>(sQ + a * kRow + t),
+                                   *reinterpret_cast<const float4 *>(sX + q * kRow + t), acc);
+                    }
+                    g1[e] += acc;
                 }
-                g1[e] = acc;
             }
         }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) atomicAdd(&grad[oW2 + (a0 + 16 * i) * kH + q0 + 16 * j], g2[i][j]);
-        const int w = tid + i * kGradThreads;
-        if (w < kH * kIn) atomicAdd(&grad[oW1 + w], g1[i]);
-    }
-    if (part == 0) {
-        atomicAdd(&grad[oB1 + row], gb1);
-        atomicAdd(&grad[oB2 + row], gb2);
-        atomicAdd(&grad[oW3 + row], gw3);
     }
     if (tid < kTile) {
         gl = warp_sum(gl);
         gb3 = warp_sum(gb3);
-        if ((tid & 31) == 0) {
-            atomicAdd(&grad[oB3], gb3);
-            atomicAdd(loss, gl);
-        }
     }
+    __syncthreads();
+    // every parameter's sum over the block's tiles in the place of the parameter
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) P[oW2 + (a0 + 16 * i) * kH + q0 + 16 * j] = g2[i][j];
+        const int w = tid + i * kGradThreads;
+        if (w < kH * kIn) P[oW1 + w] = g1[i];
+    }
+    if (part == 0) {
+        P[oB1 + row] = gb1;
+        P[oB2 + row] = gb2;
+        P[oW3 + row] = gw3;
+    }
+    if (tid == 32) {
+        sz[0][0] = gl;
+        sz[0][1] = gb3;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        P[kParams] = gl + sz[0][0];
+        P[oB3] = gb3 + sz[0][1];
+    }
+    cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    const int q = (int)cluster.block_rank() * kGradThreads + tid;
+    if (q <= kParams) {
+        float v[kGradCluster];
+#pragma unroll
+        for (int r = 0; r < kGradCluster; ++r) v[r] = cluster.map_shared_rank(P, r)[q];
+        atomicAdd(q < kParams ? &grad[q] : loss,
+                  ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7])));
+    }
+    cluster.sync();  // a block's shared memory stays until the others have read it
 }
 
 // Adam (Kingma & Ba 2015) on the summed gradient times `scale`
@@ -696,9 +730,10 @@ int acfd_mlp_grad(const float *params, const float *X, const float *Y, int n, fl
         return ACFD_ERR_ARG;
     }
     if (n == 0) return ACFD_OK;
-    const int tiles = (n - 1) / acfd::sensor::kTile + 1;
-    acfd::sensor::mlp_grad_kernel<<<std::min(tiles, acfd::sensor::kGradBlocks), acfd::sensor::kGradThreads, 0,
-                                    (cudaStream_t)stream>>>(params, X, Y, n, pos_weight, grad, loss);
+    namespace sn = acfd::sensor;
+    const int tiles = (n - 1) / sn::kTile + 1;
+    const int clusters = (std::min(tiles, sn::kGradBlocks) + sn::kGradCluster - 1) / sn::kGradCluster;
+    sn::mlp_grad_kernel<<<clusters * sn::kGradCluster, sn::kGradThreads, 0, (cudaStream_t)stream>>>(params, X, Y, n, pos_weight, grad, loss);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? ACFD_OK : acfd::cuda_status(e, "mlp_grad launch");
 }
