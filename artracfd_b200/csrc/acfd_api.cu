@@ -3048,7 +3048,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
             b->persist_blocks = bps * b->sms;
             b->persist_ok = true;
             // available (acfd_batch_set_kernel), not the default: measured
-            // 859 against 911 Mcell-steps/s for one launch per RK stage on the
+            // 859 against 999 Mcell-steps/s for one launch per RK stage on the
             // 48-case batch
             b->persist = false;
         } else {
