@@ -1033,8 +1033,8 @@ int discretize(acfd_case *cs, double dt_scale, int s, int next = 3, bool push = 
 
 // the X half steps may run as Y sweeps of the transposed state (build_xt):
 // the FP32 forms, whose X sweep is slower than the Y sweep by more than the
-// two transposes of U[TO] cost (the fast FP64 form's is not: TGV 128^3, 12 us
-// a stage, 72 us a step, against 80 us of transposes), no bodies (whose ghost
+// two transposes of U[TO] cost (the fast FP64 form's is not: TGV 128^3, 14 us
+// a stage, 84 us a step, against 80 us of transposes), no bodies (whose ghost
 // values follow the fill), no debug scans
 bool xt_eligible(const acfd_case *cs)
 {
