@@ -153,10 +153,11 @@ struct StepPiece {
 };
 
 // tensor maps of the FP64 line march along one axis: a plane of U[tn] with
-// its halo and the tile's plane of U[to], with the extents they were encoded for
+// its halo and the tile's plane of U[to], and the tile with the cuts of each
+// plane variant
 struct LineMaps {
     CUtensorMap map, omap;
-    int BXp = 0, BC = 0, OX = 0, NR = 0;
+    LineTile tile[kPlaneVariants];
     bool ok = false;
 };
 
@@ -311,7 +312,10 @@ int encode_box_map(const Grid &g, double *U, const int b[3], CUtensorMap *out, i
 // maps.ok stays false where no tile fits
 int encode_line_maps(const Grid &g, double *U, int s, bool visc, int sms, LineMaps &maps)
 {
-    const LineTile lt = line_tile(g, s, visc, 1, sms, true);
+    for (int v = 0; v < kPlaneVariants; ++v) {
+        maps.tile[v] = line_tile(g, s, visc, kPlaneWaves[v], sms, kPlaneShare[v]);
+    }
+    const LineTile &lt = maps.tile[0];  // the same tile in all of them
     if (lt.pt.NR < 1 || lt.pt.BC > 256) {
         return ACFD_OK;
     }
@@ -320,10 +324,6 @@ int encode_line_maps(const Grid &g, double *U, int s, bool visc, int sms, LineMa
     int st = encode_box_map(g, U, box, &maps.map, 1);
     if (st == ACFD_OK) st = encode_box_map(g, U, obox, &maps.omap, 1);
     if (st != ACFD_OK) return st;
-    maps.BXp = lt.pt.BXp;
-    maps.BC = lt.pt.BC;
-    maps.OX = lt.OX;
-    maps.NR = lt.pt.NR;
     maps.ok = true;
     return ACFD_OK;
 }
@@ -331,14 +331,11 @@ int encode_line_maps(const Grid &g, double *U, int s, bool visc, int sms, LineMa
 // one FP64 stage on the line march, the launch cut as plane variant v asks
 int line_stage(const acfd_case *cs, const Grid &g, const StageArgs &a, int s, int v, const LineMaps &maps)
 {
-    const bool visc = viscous(cs);
-    const LineTile lt = line_tile(g, s, visc, kPlaneWaves[v - kPlaneFirst], cs->sms, kPlaneShare[v - kPlaneFirst]);
-    if (!maps.ok || lt.pt.BXp != maps.BXp || lt.pt.BC != maps.BC || lt.OX != maps.OX || lt.pt.NR != maps.NR) {
-        set_error("line tile (%d x %d) does not match its encoded box (%d x %d)", lt.pt.BXp, lt.pt.BC, maps.BXp,
-                  maps.BC);
+    if (!maps.ok) {
+        set_error("no line tile fits axis %d", s);
         return ACFD_ERR_STATE;
     }
-    return launch_stage_line(g, cs->mp, a, s, visc, lt, maps.map, maps.omap, cs->stream);
+    return launch_stage_line(g, cs->mp, a, s, viscous(cs), maps.tile[v - kPlaneFirst], maps.map, maps.omap, cs->stream);
 }
 
 int encode_state_maps(acfd_case *cs)
