@@ -109,7 +109,7 @@ constexpr int kPlaneVariants = 6;
 constexpr int kPlaneWaves[kPlaneVariants] = {1, 2, 4, 1, 2, 4};
 constexpr bool kPlaneShare[kPlaneVariants] = {false, false, false, true, true, true};
 constexpr int kPlaneFirst = kTileVariants + kMarchVariants;
-constexpr long long kLineDefaultNodes = 1 << 17, kShareDefaultNodes = 1 << 19;  // computed nodes (acfd_init)
+constexpr long long kLineDefaultNodes = 1 << 17;  // computed nodes (fp64_defaults)
 constexpr int kStageVariants = kPlaneFirst + kPlaneVariants;
 static_assert(ACFD_BRICK_VARIANTS == kTileVariants && ACFD_STAGE_VARIANTS == kStageVariants &&
                   ACFD_PLANE_VARIANT == kPlaneFirst,
@@ -390,6 +390,49 @@ int encode_state_maps(acfd_case *cs)
         if (st != ACFD_OK) return st;
     }
     return ACFD_OK;
+}
+
+// The variants that the FP64 form starts on (acfd_autotune times them all).  Below
+// kLineDefaultNodes the first brick, whose stages write their own ghost copies
+// (ensure_push): a step of 33^3 nodes takes 183 us there, 255 in segments.  From
+// there, each axis on its own, the line march where its iterations
+// (line_iterations), in segments or in shares, cost less than the brick's tiles of
+// 240 nodes: an iteration of one consumer warp on every SM takes as long as the
+// chip needs for 14 to 15 tiles (inviscid: 2.3-2.4 us against 13 ns a tile and
+// twelve warps) or 13.5 (viscous: 2.0-2.8 us, 17.5 ns, eight or twelve warps); the
+// rule says 14 and 12, the brick's last wave being the fuller one.  Grids that
+// leave the march's lanes empty stay on the brick: steps on the line march and on
+// the brick, us, 512 x 512 cells in a plane 434 and 335, 1 x 200,000 x 1 cells
+// 18,270 and 1,450 (the march has one line); 700 x 300 x 2 cells 597 and 1,152.
+// With the sweeps unsplit (multidim) the later axes add to U[tm], which the march
+// loads in its iterations, and those take 1.6 (inviscid) to 1.9 times as long (steps
+// of 129^3 nodes on the brick and in shares: 2,490 and 2,840 us inviscid, 3,510 and
+// 4,040 viscous, where split ones take 2,540 and 2,050, 3,630 and 2,540).
+void fp64_defaults(acfd_case *cs)
+{
+    const Grid &g = cs->grid;
+    const long long pin = pin_nodes(g);
+    if (pin < kLineDefaultNodes || !cs->pmaps_ok) return;
+    const bool visc = viscous(cs);
+    for (int s = 0; s < 3; ++s) {
+        if (!cs->line[s].ok) continue;
+        const int Ls = s == 0 ? g.hi[1] - g.lo[1] : g.hi[s] - g.lo[s];
+        const long long seg = line_iterations(cs->line[s].tile[0], Ls, cs->sms);
+        const long long share = line_iterations(cs->line[s].tile[3], Ls, cs->sms);
+        int step[3];
+        long long tiles = 1;
+        bool launchable = true;  // blocks of the brick's grid along y and z
+        brick_step(s, visc, 0, step);
+        for (int a = 0; a < 3; ++a) {
+            const int n = (g.hi[a] - g.lo[a] + step[a] - 1) / step[a];
+            tiles *= n;
+            if (a > 0 && n > 65535) launchable = false;
+        }
+        long long cost = std::min(seg, share) * line_shape(s == 0, visc).warps * (visc ? 12 : 14);  // in tiles
+        if (cs->model.multidim == 1 && s != 0) cost = cost * 7 / 4;
+        if (launchable && cost > tiles) continue;
+        cs->tile_var[ACFD_FP64][s] = kPlaneFirst + (seg <= share ? 0 : 3);
+    }
 }
 
 // read and clear the device error word
@@ -1548,16 +1591,6 @@ static int init_case(const acfd_partition_t *part, const acfd_model_t *model, bo
     }
     g.pitch = (part->n[0] + 7) & ~7;
     g.nn = (long long)g.pitch * g.n[1] * g.n[2];
-    // The FP64 form starts on the line march where it is faster than the brick,
-    // cut into segments below the nodes where equal shares are faster.  Step
-    // times on the brick, the segments and the shares, us: 33^3 nodes 228 / 255 /
-    // 576, 96x62x34 (WENO3) 297 / 284 / 354, 65^3 664 / 571 / 644, 89x69x49 631 /
-    // 589 / 650, 158x96x60 1,545 / 1,387 / 1,328, 7.1 M nodes around bodies 11,415
-    // / 14,616 / 8,675
-    const long long pin = pin_nodes(g);
-    if (pin >= kLineDefaultNodes) {
-        for (int s = 0; s < 3; ++s) cs->tile_var[ACFD_FP64][s] = kPlaneFirst + (pin >= kShareDefaultNodes ? 3 : 0);
-    }
     ModelParams &m = cs->mp;
     m.gamma = model->gamma;
     m.gasR = model->gasR;
@@ -1606,6 +1639,7 @@ static int init_case(const acfd_partition_t *part, const acfd_model_t *model, bo
         acfd_finalize(cs);
         return st;
     }
+    fp64_defaults(cs);
     if (getenv("ACFD_PLAIN_KERNELS")) {
         cs->plain_kernels = true;
     }

@@ -168,11 +168,12 @@ int acfd_synchronize(acfd_case_t *cs);
  * waves of resident warps; ACFD_PLANE_VARIANT .. ACFD_STAGE_VARIANTS-1 the
  * plane-march kernels (a TMA ring of halo'd planes) with 1, 2 or 4 waves of
  * blocks, first with each tile's lines cut into equal segments, then with
- * equal shares of all tiles' planes per block.  The choice is kept per arithmetic form; the FP32 forms start on the
- * brick for X and the 4-wave plane march for Y and Z, the FP64 form on the
- * first brick below 131,072 computed nodes and on the plane march with one wave
- * from there (segments; equal shares from 524,288 nodes); acfd_autotune replaces these with the measured
- * fastest. */
+ * equal shares of all tiles' planes per block.  The choice is kept per
+ * arithmetic form; the FP32 forms start on the brick for X and the 4-wave plane
+ * march for Y and Z.  The FP64 form starts on the first brick below 131,072
+ * computed nodes; from there each axis starts on the plane march with one wave
+ * (segments or equal shares) or on the first brick, whichever the grid's extents
+ * fill better.  acfd_autotune replaces these with the measured fastest. */
 #define ACFD_BRICK_VARIANTS 2
 #define ACFD_PLANE_VARIANT 5
 #define ACFD_STAGE_VARIANTS 11
