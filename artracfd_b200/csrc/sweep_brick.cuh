@@ -272,7 +272,11 @@ __device__ __forceinline__ void push_copies(const StageArgs &a, long long nn, in
 // The caller has initialised the block's mbarrier; `parity` is the phase this
 // tile's load completes.  Returns false when the load did not complete within
 // the wait limit (the block must then stop).
-template <int S, int NP, bool VISC, bool HYB, int VAR>
+// PUSH: the stage writes its nodes' ghost copies itself (FP64 form).  A kernel of
+// its own: behind a test in the one kernel the copies cost the stages that write
+// none 1.5 to 5% with WENO3 (RK2 steps of 52^3, 60^3 and 90^3 cells, inviscid: 138,
+// 164 and 428 us in one kernel, 130, 156 and 405 in two).
+template <int S, int NP, bool VISC, bool HYB, int VAR, bool PUSH>
 __device__ __forceinline__ bool brick_tile(const Grid &g, const ModelParams &mp, const StageArgs &a,
                                            const CUtensorMap *map, int tbx, int tby, int tbz, unsigned char *smem,
                                            uint32_t parity)
@@ -343,9 +347,9 @@ __device__ __forceinline__ bool brick_tile(const Grid &g, const ModelParams &mp,
         }
     }
     const double rdt = (a.dt_scale * a.dt[0]) * g.dd[S];
-    int4 push = make_int4(-1, -1, -1, -1);  // the node's ghost copies (FP64 form)
-    if constexpr (sizeof(Real) == sizeof(double)) {
-        if (a.push && inside && q >= 0 && sl >= 1) {
+    int4 push = make_int4(-1, -1, -1, -1);  // the node's ghost copies
+    if constexpr (PUSH) {
+        if (inside && q >= 0 && sl >= 1) {
             const int at = a.push[node];
             if (at >= 0) push = a.push_list[at];
         }
@@ -443,7 +447,7 @@ __device__ __forceinline__ bool brick_tile(const Grid &g, const ModelParams &mp,
     __syncthreads();
 
     // C. node update
-    if constexpr (sizeof(Real) == sizeof(double)) {
+    if constexpr (PUSH) {
         if (upd || push.x >= 0) {
             const int lt = tid - ((S == 0) ? 1 : (S == 1 ? B::TX : B::TX * B::TY));
             const int c = bidx(i, j, k);
@@ -487,7 +491,7 @@ __device__ __forceinline__ bool brick_tile(const Grid &g, const ModelParams &mp,
 }
 
 // one tile per block
-template <int S, int NP, bool VISC, bool HYB, int VAR>
+template <int S, int NP, bool VISC, bool HYB, int VAR, bool PUSH>
 __global__ void __launch_bounds__(kBrickThreads, 2)
 stage_brick(Grid g, ModelParams mp, StageArgs a, const __grid_constant__ CUtensorMap map)
 {
@@ -499,10 +503,10 @@ stage_brick(Grid g, ModelParams mp, StageArgs a, const __grid_constant__ CUtenso
     }
     __syncthreads();
     pdl_wait();
-    brick_tile<S, NP, VISC, HYB, VAR>(g, mp, a, &map, blockIdx.x, blockIdx.y, blockIdx.z, smem, 0);
+    brick_tile<S, NP, VISC, HYB, VAR, PUSH>(g, mp, a, &map, blockIdx.x, blockIdx.y, blockIdx.z, smem, 0);
 }
 
-template <int S, int NP, bool VISC, bool HYB, int VAR>
+template <int S, int NP, bool VISC, bool HYB, int VAR, bool PUSH>
 static int launch_brick_one(const Grid &g, const ModelParams &m, const StageArgs &a, cudaStream_t st)
 {
     typedef Brick<S, VISC, VAR> B;
@@ -511,7 +515,7 @@ static int launch_brick_one(const Grid &g, const ModelParams &m, const StageArgs
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev >= 0 && dev < 64 && !configured[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(stage_brick<S, NP, VISC, HYB, VAR>,
+        cudaError_t e = cudaFuncSetAttribute(stage_brick<S, NP, VISC, HYB, VAR, PUSH>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, LY::total);
         if (e != cudaSuccess) return cuda_status(e, "cudaFuncSetAttribute(stage_brick)");
         configured[dev] = true;
@@ -519,7 +523,7 @@ static int launch_brick_one(const Grid &g, const ModelParams &m, const StageArgs
     const int L0 = g.hi[0] - g.lo[0], L1 = g.hi[1] - g.lo[1], L2 = g.hi[2] - g.lo[2];
     dim3 grid((L0 + B::SX - 1) / B::SX, (L1 + B::SY - 1) / B::SY, (L2 + B::SZ - 1) / B::SZ);
     dim3 block(B::TX, B::TY, B::TZ);
-    cudaError_t e = launch_k(stage_brick<S, NP, VISC, HYB, VAR>, grid, block, LY::total, st, g, m, a,
+    cudaError_t e = launch_k(stage_brick<S, NP, VISC, HYB, VAR, PUSH>, grid, block, LY::total, st, g, m, a,
                              a.maps[S * kTileVariants + VAR]);
     return e == cudaSuccess ? ACFD_OK : cuda_status(e, "stage_brick launch");
 }
@@ -527,8 +531,14 @@ static int launch_brick_one(const Grid &g, const ModelParams &m, const StageArgs
 template <int S, int NP, bool VISC, bool HYB>
 static int launch_brick_var(const Grid &g, const ModelParams &m, const StageArgs &a, cudaStream_t st)
 {
-    if (a.var[S] == 1) return launch_brick_one<S, NP, VISC, HYB, 1>(g, m, a, st);
-    return launch_brick_one<S, NP, VISC, HYB, 0>(g, m, a, st);
+    if constexpr (sizeof(Real) == sizeof(double)) {
+        if (a.push) {
+            return a.var[S] == 1 ? launch_brick_one<S, NP, VISC, HYB, 1, true>(g, m, a, st)
+                                 : launch_brick_one<S, NP, VISC, HYB, 0, true>(g, m, a, st);
+        }
+    }
+    return a.var[S] == 1 ? launch_brick_one<S, NP, VISC, HYB, 1, false>(g, m, a, st)
+                         : launch_brick_one<S, NP, VISC, HYB, 0, false>(g, m, a, st);
 }
 
 template <int NP, bool VISC, bool HYB>
@@ -617,7 +627,7 @@ stage_batch(const BatchCase *cases, const CUtensorMap *maps, const long long *pr
         a.status = status;
         a.flags = C.flags;
         a.wait_limit = kWaitLimitDefault;
-        if (!brick_tile<S, 6, true, HYB, 0>(C.g, C.mp, a, maps + 3 * lo + S, tx, ty, tz, smem, parity)) {
+        if (!brick_tile<S, 6, true, HYB, 0, false>(C.g, C.mp, a, maps + 3 * lo + S, tx, ty, tz, smem, parity)) {
             break;
         }
         parity ^= 1u;
