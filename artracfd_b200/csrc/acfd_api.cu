@@ -1252,7 +1252,7 @@ int ensure_push(acfd_case *cs)
 
 bool use_push(const acfd_case *cs, int s)
 {
-    return cs->push_state == 1 && may_push(cs, s) && !cs->prof;
+    return cs->push_state == 1 && may_push(cs, s);
 }
 
 // EvolveFluidDynamics (fluid_dynamics.c:55-116); the step dt is in d_dt
@@ -1861,6 +1861,7 @@ int acfd_profile_step(acfd_case_t *cs, double dt, int cap, int *kind, int *axis,
         set_error("acfd_profile_step: bad output arrays");
         return ACFD_ERR_ARG;
     }
+    TRY(ensure_push(cs));
     std::vector<StepPiece> pieces;
     cs->prof = &pieces;
     int st = set_dt(cs, dt);

@@ -358,7 +358,9 @@ def _stage_profile(torch, s, spec, nodes_pin, stream, per_axis=None, other=None)
             bc_ms.append(ms)
         elif other is not None:
             other.setdefault(names.get(kind, str(kind)), []).append(ms)
-    return sum(stage_ms) / len(stage_ms), sum(bc_ms) / len(bc_ms), sum(stage_bytes) / len(stage_bytes)
+    # no fill pieces where the stages write their ghost copies themselves
+    bc = sum(bc_ms) / len(bc_ms) if bc_ms else 0.0
+    return sum(stage_ms) / len(stage_ms), bc, sum(stage_bytes) / len(stage_bytes)
 
 
 def _pin_mask(part):

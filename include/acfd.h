@@ -259,7 +259,9 @@ int acfd_evolve_fluid_graph(acfd_case_t *cs, double dt);
 /* Pieces of a time step, as acfd_profile_step reports them. */
 #define ACFD_PIECE_STAGE 0     /* an LLLU stage kernel along sweep axis[i] */
 #define ACFD_PIECE_STAGE_XT 1  /* an LLLU stage along x, run as the Y sweep of the transposed state */
-#define ACFD_PIECE_FILL 2      /* the ghost fill (TreatBoundary) after a stage */
+#define ACFD_PIECE_FILL 2      /* the ghost fill (TreatBoundary) after a stage; none where the stage
+                                * writes its ghost copies itself (FP64 form on the brick kernels,
+                                * small grids whose fill is copies) */
 #define ACFD_PIECE_TRANSPOSE 3 /* U[TO] or the x flags to or from the transposed state */
 #define ACFD_PIECE_SENSOR 4    /* the learned sensor's flags of U[TO] */
 /* acfd_evolve_fluid with CUDA events around each piece of the step on the
