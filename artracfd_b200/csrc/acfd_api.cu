@@ -1953,9 +1953,19 @@ int acfd_autotune(acfd_case_t *cs, int tiles[3])
                 st = launch_transpose_u8(cs->sensor_flags, cs->grid, cs->xfl + cs->xg.nn, cs->xg, cs->stream);
             }
         }
-        auto run = [&](double coeA, double coeB, int tn, int tm) {
-            return xt ? stage_xt(cs, 1.0, coeA, coeB, ACFD_TO, tn, tm)
-                      : stage(cs, 1.0, coeA, coeB, ACFD_TO, tn, tm, s);
+        // where the brick stages write their ghost copies themselves, every other
+        // stage is timed with the fill that follows it (a third of a stage of 32^3
+        // cells); elsewhere all variants have the same fill, and it is left out
+        const int var0 = var_of[s];
+        var_of[s] = 0;
+        st = st == ACFD_OK ? ensure_push(cs) : st;
+        const bool fills = !xt && use_push(cs, s);
+        var_of[s] = var0;
+        auto run = [&](double coeA, double coeB, int tn, int tm) -> int {
+            if (xt) return stage_xt(cs, 1.0, coeA, coeB, ACFD_TO, tn, tm);
+            const bool push = fills && use_push(cs, s);
+            TRY(stage(cs, 1.0, coeA, coeB, ACFD_TO, tn, tm, s, push ? s : -1));
+            return fills && !push ? treat_boundary(cs, tm, s) : ACFD_OK;
         };
         float best = 1e30f;
         int best_var = var_of[s];
@@ -1991,6 +2001,12 @@ int acfd_autotune(acfd_case_t *cs, int tiles[3])
     }
     release_graph(cs);
     TRY(check_device_status(cs));
+    if (cs->push_state == 1 && !(may_push(cs, 0) || may_push(cs, 1) || may_push(cs, 2))) {
+        cudaFree(cs->push);  // built for the timing alone
+        cs->push = nullptr;
+        cs->push_list = nullptr;
+        cs->push_state = 0;
+    }
     for (int s = 0; s < 3; ++s) {
         if (tiles) tiles[s] = var_of[s];
     }

@@ -181,7 +181,8 @@ int acfd_synchronize(acfd_case_t *cs);
  * case's current state (RK stage 2, reading U[TO] and U[TN] and writing
  * U[TM], after a stage 1 into U[TN]; both are overwritten by every step) for
  * the current arithmetic form and keeps the fastest; tiles[3] (optional)
- * receives the chosen variant per axis. */
+ * receives the chosen variant per axis.  A variant whose stages need a ghost
+ * fill after them is timed with it where others do without. */
 int acfd_autotune(acfd_case_t *cs, int tiles[3]);
 /* Select the stage-kernel variant of each sweep axis for the current
  * arithmetic form (tests and experiments; acfd_autotune picks by timing). */
