@@ -218,6 +218,7 @@ def load_library(path: str | None = None):
         "acfd_batch_set_precision": [vp, i],
         "acfd_batch_sensor_load": [vp, ctypes.POINTER(ctypes.c_float), ctypes.c_float],
         "acfd_batch_advance": [vp, dp, i, dp],
+        "acfd_batch_transposed": [vp, ctypes.POINTER(ctypes.c_int)],
         "acfd_batch_stats": [vp, ctypes.POINTER(ctypes.c_longlong)],
         "acfd_batch_set_stream": [vp, vp],
         "acfd_batch_set_kernel": [vp, i],

@@ -127,6 +127,13 @@ class Batch:
                                           dts.ctypes.data_as(ctypes.POINTER(ctypes.c_double))), self.lib)
         return dts[:steps]
 
+    def transposed(self) -> bool:
+        """Whether the next step runs the X half steps on transposed states
+        (acfd_batch_transposed)."""
+        on = ctypes.c_int()
+        check(self.lib.acfd_batch_transposed(self.h, ctypes.byref(on)), self.lib)
+        return bool(on.value)
+
     def launches(self) -> int:
         n = ctypes.c_longlong()
         check(self.lib.acfd_batch_stats(self.h, ctypes.byref(n)), self.lib)

@@ -161,6 +161,27 @@ struct LineMaps {
     bool ok = false;
 };
 
+// Use of the transposed levels of a batch, by the batch or one of its cases'
+// handles: they stay until it ends (give_back_batch_levels).
+thread_local bool t_uses_batch_levels = false;
+struct BatchLevelsUse {
+    std::mutex *m;
+    explicit BatchLevelsUse(std::mutex *lock) : m(lock)
+    {
+        if (!m) return;
+        m->lock();
+        t_uses_batch_levels = true;
+    }
+    ~BatchLevelsUse()
+    {
+        if (!m) return;
+        t_uses_batch_levels = false;
+        m->unlock();
+    }
+    BatchLevelsUse(const BatchLevelsUse &) = delete;
+    BatchLevelsUse &operator=(const BatchLevelsUse &) = delete;
+};
+
 struct acfd_case {
     acfd_partition_t part;
     acfd_model_t model;
@@ -228,7 +249,8 @@ struct acfd_case {
     // the copy-only fills remapped to it (xbc: for the next stage's sweep axis,
     // or every ghost node).
     bool xt_ok = false;
-    bool xt_batch = false;         // the transposed levels belong to a batch's step alone
+    bool xt_batch = false;         // the transposed levels belong to a batch's step alone ...
+    std::mutex *xt_lock = nullptr; // ... which may give them back (BatchLevelsUse)
     bool xt_all_forms = false;     // the transposed X sweep for the fast FP64 form too
     Grid xg = {};
     double *xU = nullptr;
@@ -557,7 +579,7 @@ bool make_fills(std::vector<int2> *const pairs[4], std::vector<int4> *const prog
         at[s][1] = put(f[s].h_single.data(), f[s].nsingle * sizeof(int2));
         at[s][2] = progs ? put(progs[s]->data(), f[s].nprog * sizeof(int4)) : 0;
     }
-    if (cudaMalloc(mem, h.size() + 16) != cudaSuccess ||
+    if (device_malloc(mem, h.size() + 16) != cudaSuccess ||
         cudaMemcpy(*mem, h.data(), h.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -1080,7 +1102,7 @@ bool xt_eligible(const acfd_case *cs)
 {
     const bool form = cs->mode == ACFD_FP32_HYBRID || cs->mode == ACFD_FP32_BULK ||
                       (cs->xt_all_forms && cs->mode == ACFD_FP64 && cs->xline.ok);
-    return cs->xt_ok && !cs->xt_batch && !cs->debug && !cs->plain_kernels && form && !(cs->ib && ib_count(cs->ib) > 0);
+    return !cs->xt_batch && cs->xt_ok && !cs->debug && !cs->plain_kernels && form && !(cs->ib && ib_count(cs->ib) > 0);
 }
 
 // ... and do, when the X sweep's variant is a plane march (acfd_autotune
@@ -1542,7 +1564,7 @@ int ensure_staging(acfd_case *cs)
         return ACFD_OK;
     }
     const size_t total = (size_t)cs->grid.n[0] * cs->grid.n[1] * cs->grid.n[2];
-    ACFD_CUDA(cudaMalloc(&cs->staging, total * sizeof(acfd_node_t)));
+    ACFD_CUDA(device_malloc(&cs->staging, total * sizeof(acfd_node_t)));
     return ACFD_OK;
 }
 
@@ -1623,15 +1645,15 @@ static int init_case(const acfd_partition_t *part, const acfd_model_t *model, bo
     cs->own_stream = true;
     const size_t ubytes = sizeof(double) * kLevels * kVars * (size_t)g.nn;
     const size_t fbytes = sizeof(int) * 4 * (size_t)g.nn;
-    if ((e = cudaMalloc(&cs->U, ubytes)) != cudaSuccess ||
-        (e = cudaMalloc(&cs->flags, fbytes)) != cudaSuccess ||
-        (e = cudaMalloc(&cs->d_dt, sizeof(double))) != cudaSuccess ||
-        (e = cudaMalloc(&cs->cfl_part, sizeof(double) * kCflPartials)) != cudaSuccess ||
+    if ((e = device_malloc(&cs->U, ubytes)) != cudaSuccess ||
+        (e = device_malloc(&cs->flags, fbytes)) != cudaSuccess ||
+        (e = device_malloc(&cs->d_dt, sizeof(double))) != cudaSuccess ||
+        (e = device_malloc(&cs->cfl_part, sizeof(double) * kCflPartials)) != cudaSuccess ||
         (e = cudaMemset(cs->cfl_part, 0, sizeof(double) * kCflPartials)) != cudaSuccess ||
-        (e = cudaMalloc(&cs->cfl_out, sizeof(double) * 4)) != cudaSuccess ||
+        (e = device_malloc(&cs->cfl_out, sizeof(double) * 4)) != cudaSuccess ||
         (e = cudaMallocHost(&cs->h_cfl, sizeof(double) * 6)) != cudaSuccess ||
-        (e = cudaMalloc(&cs->dstatus, sizeof(int))) != cudaSuccess ||
-        (e = cudaMalloc(&cs->bcbar, 2 * sizeof(unsigned))) != cudaSuccess) {
+        (e = device_malloc(&cs->dstatus, sizeof(int))) != cudaSuccess ||
+        (e = device_malloc(&cs->bcbar, 2 * sizeof(unsigned))) != cudaSuccess) {
         st = cuda_status(e, "acfd_init allocation");
         acfd_finalize(cs);
         return st;
@@ -1655,7 +1677,7 @@ static int init_case(const acfd_partition_t *part, const acfd_model_t *model, bo
     {
         const char *dbg = getenv("ACFD_DEBUG");
         if (dbg && atoi(dbg) != 0) {
-            if ((e = cudaMalloc(&cs->dbg_word, sizeof(int))) != cudaSuccess ||
+            if ((e = device_malloc(&cs->dbg_word, sizeof(int))) != cudaSuccess ||
                 (e = cudaMemsetAsync(cs->dbg_word, 0, sizeof(int), cs->stream)) != cudaSuccess) {
                 st = cuda_status(e, "acfd_init (debug word)");
                 acfd_finalize(cs);
@@ -1781,8 +1803,10 @@ int acfd_sync_to_device(acfd_case_t *cs, const acfd_node_t *node, unsigned mask)
     TRY(launch_scatter_nodes(cs->grid, cs->staging, cs->U, cs->flags, mask, cs->stream));
     if (mask & ACFD_SYNC_FLAGS) {
         TRY(ib_flags_changed(cs->ib, cs->grid, cs->mp, cs->part, cs->flags, cs->stream));
+        BatchLevelsUse use(cs->xt_lock);
         if (cs->xt_ok) {
             TRY(launch_transpose_int(cs->flags, cs->grid, cs->xdid, cs->xg, cs->stream));  // the node types
+            ACFD_CUDA(cudaStreamSynchronize(cs->stream));
         }
     }
     ACFD_CUDA(cudaStreamSynchronize(cs->stream));
@@ -2050,10 +2074,10 @@ int acfd_sensor_load(acfd_case_t *cs, const float *params, float threshold)
     }
     const int np = sensor_param_count();
     if (!cs->sensor_params) {
-        ACFD_CUDA(cudaMalloc(&cs->sensor_params, sizeof(float) * np));
-        ACFD_CUDA(cudaMalloc(&cs->sensor_flags, (size_t)3 * cs->grid.nn));
-        ACFD_CUDA(cudaMalloc(&cs->sensor_rp, sizeof(float2) * cs->grid.nn));
-        ACFD_CUDA(cudaMalloc(&cs->sensor_count, sizeof(unsigned long long)));
+        ACFD_CUDA(device_malloc(&cs->sensor_params, sizeof(float) * np));
+        ACFD_CUDA(device_malloc(&cs->sensor_flags, (size_t)3 * cs->grid.nn));
+        ACFD_CUDA(device_malloc(&cs->sensor_rp, sizeof(float2) * cs->grid.nn));
+        ACFD_CUDA(device_malloc(&cs->sensor_count, sizeof(unsigned long long)));
     }
     ACFD_CUDA(cudaMemcpyAsync(cs->sensor_params, params, sizeof(float) * np, cudaMemcpyHostToDevice, cs->stream));
     ACFD_CUDA(cudaMemsetAsync(cs->sensor_flags, 1, (size_t)3 * cs->grid.nn, cs->stream));
@@ -2200,8 +2224,12 @@ int acfd_geo_upload(acfd_case_t *cs, const acfd_polyhedron_t *poly, int totN)
     }
     // bodies change the node types through their treatment: the X half steps
     // stay on the X sweep from now on
-    const bool leave_xt = totN > 0 && cs->xt_ok;
-    if (totN > 0) cs->xt_ok = false;
+    bool leave_xt = false;
+    if (totN > 0) {
+        BatchLevelsUse use(cs->xt_lock);
+        leave_xt = cs->xt_ok;
+        cs->xt_ok = false;
+    }
     bool relayout = true;
     TRY(ib_upload(cs->ib, poly, totN, cs->part, cs->stream, &relayout));
     // bodies moved in place keep every device pointer and launch shape of a
@@ -2271,7 +2299,7 @@ int acfd_snapshot_begin(acfd_case_t *cs)
     TRY(check_case(cs));
     const size_t total = node_count(cs);
     if (!cs->snap_dev) {
-        ACFD_CUDA(cudaMalloc(&cs->snap_dev, total * sizeof(acfd_node_t)));
+        ACFD_CUDA(device_malloc(&cs->snap_dev, total * sizeof(acfd_node_t)));
         ACFD_CUDA(cudaMallocHost(&cs->snap_host, total * sizeof(acfd_node_t)));
         ACFD_CUDA(cudaStreamCreateWithFlags(&cs->snap_stream, cudaStreamNonBlocking));
         ACFD_CUDA(cudaEventCreateWithFlags(&cs->snap_gathered, cudaEventDisableTiming));
@@ -2449,8 +2477,8 @@ int acfd_weno_batch(int scheme, int mode, const double *F, double *Fhat, int cou
         return ACFD_ERR_ARG;
     }
     double *dF = nullptr, *dO = nullptr;
-    ACFD_CUDA(cudaMalloc(&dF, sizeof(double) * 25 * (size_t)(count ? count : 1)));
-    cudaError_t e = cudaMalloc(&dO, sizeof(double) * 5 * (size_t)(count ? count : 1));
+    ACFD_CUDA(device_malloc(&dF, sizeof(double) * 25 * (size_t)(count ? count : 1)));
+    cudaError_t e = device_malloc(&dO, sizeof(double) * 5 * (size_t)(count ? count : 1));
     if (e != cudaSuccess) {
         cudaFree(dF);
         return cuda_status(e, "cudaMalloc");
@@ -2480,8 +2508,8 @@ int acfd_fhat_batch(const acfd_model_t *model, int s, int mode, const double *Us
     }
     const ModelParams m = params_of(model);
     double *dU = nullptr, *dO = nullptr;
-    ACFD_CUDA(cudaMalloc(&dU, sizeof(double) * 30 * (size_t)(count ? count : 1)));
-    cudaError_t e = cudaMalloc(&dO, sizeof(double) * 5 * (size_t)(count ? count : 1));
+    ACFD_CUDA(device_malloc(&dU, sizeof(double) * 30 * (size_t)(count ? count : 1)));
+    cudaError_t e = device_malloc(&dO, sizeof(double) * 5 * (size_t)(count ? count : 1));
     if (e != cudaSuccess) {
         cudaFree(dU);
         return cuda_status(e, "cudaMalloc");
@@ -2544,6 +2572,8 @@ struct acfd_batch {
     int pthreads[3] = {0, 0, 0}, psmem[3] = {0, 0, 0};
     // the X half steps as Y sweeps of the transposed states (build_batch_xt)
     bool xt_ok = false;
+    std::mutex xt_use;                     // held while a call may use the transposed levels
+    int device = 0;
     BatchCase *d_xcases = nullptr;         // [ncase]
     BatchPlane *d_xplanes = nullptr;       // [ncase][3], entry 1
     CUtensorMap *d_xpmaps = nullptr;       // [ncase][3], entry 1
@@ -2593,7 +2623,7 @@ int upload_batch_fill(BatchFill &f, const std::vector<int4> &tasks, const std::v
     f.nsingle = (int)single.size();
     if (f.ntask + f.nsingle == 0) return ACFD_OK;
     f.per_warp = run_per_warp(tasks);
-    ACFD_CUDA(cudaMalloc(&f.tasks, sizeof(int4) * ((size_t)f.ntask + f.nsingle)));
+    ACFD_CUDA(device_malloc(&f.tasks, sizeof(int4) * ((size_t)f.ntask + f.nsingle)));
     f.single = f.tasks + f.ntask;
     ACFD_CUDA(cudaMemcpy(f.tasks, tasks.data(), sizeof(int4) * f.ntask, cudaMemcpyHostToDevice));
     ACFD_CUDA(cudaMemcpy(f.single, single.data(), sizeof(int4) * f.nsingle, cudaMemcpyHostToDevice));
@@ -2641,8 +2671,10 @@ bool to_device(T *&p, const std::vector<T> &h)
 // states, as in the single case (build_xt), when every case's fill is copies: the
 // X launch of ten viscous cases of 64..128 cells a side takes 597 us against 374
 // for Y, and their step 10.23 ms with the X launches, 9.29 ms with the transposes
-// (one launch over all cases each way).  The transposed levels double a case's state, so they are held only if
-// that leaves half of the free memory; without them the X sweep stays.
+// (one launch over all cases each way).  The transposed levels double a case's
+// state, so they are held only where they take at most half of the free memory
+// and a quarter of the device's, and they go back when the library runs out of
+// device memory (give_back_batch_levels); without them the X sweep stays.
 void build_batch_xt(acfd_batch *b)
 {
     const int ncase = (int)b->cases.size();
@@ -2651,7 +2683,7 @@ void build_batch_xt(acfd_batch *b)
         need += (sizeof(double) * kLevels * kVars + sizeof(int) + 2) * (size_t)((cs->grid.n[1] + 7) & ~7) *
                 cs->grid.n[0] * cs->grid.n[2];
     }
-    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 2) {
+    if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess || need > free_b / 2 || need > total_b / 4) {
         cudaGetLastError();
         return;
     }
@@ -2659,6 +2691,7 @@ void build_batch_xt(acfd_batch *b)
     for (acfd_case *cs : b->cases) {
         build_xt(cs);
         cs->xt_batch = true;
+        cs->xt_lock = &b->xt_use;
         if (!cs->xt_ok || cudaStreamSynchronize(cs->stream) != cudaSuccess) {
             cudaGetLastError();
             release_batch_xt(b);
@@ -2728,6 +2761,39 @@ void build_batch_xt(acfd_batch *b)
         return;
     }
     b->xt_ok = true;
+}
+
+// the batches of the process that may hold transposed levels
+struct BatchList {
+    std::mutex lock;
+    std::vector<acfd_batch *> all;
+};
+BatchList &batch_list()
+{
+    static BatchList *list = new BatchList();  // not destroyed: handles may outlive static objects
+    return *list;
+}
+
+// The transposed levels of the batches on this device go back to it, each batch's
+// when no call uses them; its next step captures the X sweep.  False when there
+// were none, or from inside such a call.
+bool give_back_batch_levels()
+{
+    int dev = -1;
+    if (t_uses_batch_levels || cudaGetDevice(&dev) != cudaSuccess) return false;
+    bool any = false;
+    BatchList &list = batch_list();
+    std::lock_guard<std::mutex> guard(list.lock);
+    for (acfd_batch *b : list.all) {
+        if (b->device != dev) continue;
+        BatchLevelsUse use(&b->xt_use);
+        if (!b->xt_ok) continue;
+        cudaStreamSynchronize(b->stream);
+        batch_release_graph(b);
+        release_batch_xt(b);
+        any = true;
+    }
+    return any;
 }
 
 // a case that was given bodies has left the transposed path (acfd_geo_upload)
@@ -2884,6 +2950,16 @@ int batch_check(const acfd_batch *b)
 
 }  // namespace
 
+cudaError_t acfd::device_malloc_bytes(void **p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back_batch_levels()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 extern "C" {
 
 int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t *models, acfd_batch_t **out)
@@ -2903,6 +2979,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
         }
     }
     acfd_batch *b = new acfd_batch();
+    cudaGetDevice(&b->device);
     b->tScheme = models[0].tScheme;
     int st = ACFD_OK;
     cudaError_t e;
@@ -3025,9 +3102,9 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
             b->pblocks[s] = pprefix[(size_t)s * (ncase + 1) + ncase];
         }
         if (b->plane_ok) {
-            if ((e = cudaMalloc(&b->d_planes, sizeof(BatchPlane) * hp.size())) != cudaSuccess ||
-                (e = cudaMalloc(&b->d_pmaps, sizeof(CUtensorMap) * hpm.size())) != cudaSuccess ||
-                (e = cudaMalloc(&b->d_pprefix, sizeof(long long) * pprefix.size())) != cudaSuccess ||
+            if ((e = device_malloc(&b->d_planes, sizeof(BatchPlane) * hp.size())) != cudaSuccess ||
+                (e = device_malloc(&b->d_pmaps, sizeof(CUtensorMap) * hpm.size())) != cudaSuccess ||
+                (e = device_malloc(&b->d_pprefix, sizeof(long long) * pprefix.size())) != cudaSuccess ||
                 (e = cudaMemcpy(b->d_planes, hp.data(), sizeof(BatchPlane) * hp.size(), cudaMemcpyHostToDevice)) !=
                     cudaSuccess ||
                 (e = cudaMemcpy(b->d_pmaps, hpm.data(), sizeof(CUtensorMap) * hpm.size(), cudaMemcpyHostToDevice)) !=
@@ -3048,7 +3125,7 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
                      (void **)&b->d_cfl, (void **)&b->d_mesh, (void **)&b->d_vmax, (void **)&b->d_counter,
                      (void **)&b->d_status, (void **)&b->d_levels, (void **)&b->d_pairs};
     for (int q = 0; q < 11 && st == ACFD_OK; ++q) {
-        if ((e = cudaMalloc(ptrs[q], nbytes[q])) != cudaSuccess) {
+        if ((e = device_malloc(ptrs[q], nbytes[q])) != cudaSuccess) {
             st = cuda_status(e, "acfd_batch_init allocation");
         }
     }
@@ -3090,14 +3167,14 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
         int bps = 0;
         const size_t nflag = (size_t)kMaxStepStages * ncase;
         if (plane_persistent_occupancy(b->visc, true, b->persist_threads, b->persist_smem, &bps) == ACFD_OK &&
-            bps >= 1 && (e = cudaMalloc(&b->d_queue, sizeof(unsigned long long))) == cudaSuccess &&
-            (e = cudaMalloc(&b->d_done, sizeof(unsigned) * nflag)) == cudaSuccess &&
-            (e = cudaMalloc(&b->d_filled, sizeof(unsigned) * nflag)) == cudaSuccess &&
-            (e = cudaMalloc(&b->d_abort, sizeof(int))) == cudaSuccess &&
-            (e = cudaMalloc(&b->d_pair_off, sizeof(long long) * off.size())) == cudaSuccess &&
+            bps >= 1 && (e = device_malloc(&b->d_queue, sizeof(unsigned long long))) == cudaSuccess &&
+            (e = device_malloc(&b->d_done, sizeof(unsigned) * nflag)) == cudaSuccess &&
+            (e = device_malloc(&b->d_filled, sizeof(unsigned) * nflag)) == cudaSuccess &&
+            (e = device_malloc(&b->d_abort, sizeof(int))) == cudaSuccess &&
+            (e = device_malloc(&b->d_pair_off, sizeof(long long) * off.size())) == cudaSuccess &&
             (e = cudaMemcpy(b->d_pair_off, off.data(), sizeof(long long) * off.size(), cudaMemcpyHostToDevice)) ==
                 cudaSuccess &&
-            (e = cudaMalloc(&b->d_fill_pre, sizeof(long long) * fpre.size())) == cudaSuccess &&
+            (e = device_malloc(&b->d_fill_pre, sizeof(long long) * fpre.size())) == cudaSuccess &&
             (e = cudaMemcpy(b->d_fill_pre, fpre.data(), sizeof(long long) * fpre.size(), cudaMemcpyHostToDevice)) ==
                 cudaSuccess) {
             b->nfill = fpre[(size_t)ncase];
@@ -3119,6 +3196,10 @@ int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t
     for (acfd_case *cs : b->cases) {
         cs->mode = ACFD_FP32_BULK;
     }
+    if (b->xt_ok) {
+        std::lock_guard<std::mutex> guard(batch_list().lock);
+        batch_list().all.push_back(b);
+    }
     *out = b;
     return ACFD_OK;
 }
@@ -3127,6 +3208,11 @@ int acfd_batch_finalize(acfd_batch_t *b)
 {
     if (!b) {
         return ACFD_OK;
+    }
+    {
+        BatchList &list = batch_list();
+        std::lock_guard<std::mutex> guard(list.lock);
+        list.all.erase(std::remove(list.all.begin(), list.all.end(), b), list.all.end());
     }
     if (b->stream) cudaStreamSynchronize(b->stream);
     batch_release_graph(b);
@@ -3178,6 +3264,7 @@ int acfd_batch_set_precision(acfd_batch_t *b, int mode)
         set_error("acfd_batch_set_precision: the batch runs ACFD_FP32_BULK or ACFD_FP32_HYBRID, not %d", mode);
         return ACFD_ERR_ARG;
     }
+    BatchLevelsUse use(&b->xt_use);
     std::vector<BatchCase> hc(b->cases.size());
     ACFD_CUDA(cudaMemcpy(hc.data(), b->d_cases, sizeof(BatchCase) * hc.size(), cudaMemcpyDeviceToHost));
     for (size_t c = 0; c < b->cases.size(); ++c) {
@@ -3215,6 +3302,7 @@ int acfd_batch_sensor_load(acfd_batch_t *b, const float *params, float threshold
     for (acfd_case *cs : b->cases) {
         TRY(acfd_sensor_load(cs, params, threshold));
     }
+    BatchLevelsUse use(&b->xt_use);
     batch_release_graph(b);
     return ACFD_OK;
 }
@@ -3227,6 +3315,7 @@ int acfd_batch_advance(acfd_batch_t *b, const double *cfl, int steps, double *dt
         set_error("acfd_batch_advance: bad arguments");
         return ACFD_ERR_ARG;
     }
+    BatchLevelsUse use(&b->xt_use);
     ACFD_CUDA(cudaMemcpyAsync(b->d_cfl, cfl, sizeof(double) * ncase, cudaMemcpyHostToDevice, b->stream));
     const bool xt = batch_use_xt(b);
     if (!b->exec || b->graph_mode != b->mode || b->graph_xt != xt) {
@@ -3287,6 +3376,7 @@ int acfd_batch_set_kernel(acfd_batch_t *b, int kernel)
         set_error("acfd_batch_set_kernel: the persistent step needs copy-only ghost fills in every case");
         return ACFD_ERR_STATE;
     }
+    BatchLevelsUse use(&b->xt_use);
     b->plane = (kernel != ACFD_BATCH_BRICK);
     b->persist = (kernel == ACFD_BATCH_PERSISTENT);
     batch_release_graph(b);
@@ -3300,11 +3390,24 @@ int acfd_batch_set_stream(acfd_batch_t *b, void *stream)
         set_error("acfd_batch_set_stream: null stream");
         return ACFD_ERR_ARG;
     }
+    BatchLevelsUse use(&b->xt_use);
     ACFD_CUDA(cudaStreamSynchronize(b->stream));
     ACFD_CUDA(cudaStreamDestroy(b->stream));
     b->stream = static_cast<cudaStream_t>(stream);
     b->own_stream = false;
     batch_release_graph(b);
+    return ACFD_OK;
+}
+
+int acfd_batch_transposed(acfd_batch_t *b, int *on)
+{
+    TRY(batch_check(b));
+    if (!on) {
+        set_error("acfd_batch_transposed: null output");
+        return ACFD_ERR_ARG;
+    }
+    BatchLevelsUse use(&b->xt_use);
+    *on = batch_use_xt(b) ? 1 : 0;
     return ACFD_OK;
 }
 

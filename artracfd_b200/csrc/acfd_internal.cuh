@@ -403,6 +403,14 @@ int sensor_param_count();
 // ---------------------------------------------------------------------------
 void set_error(const char *fmt, ...);
 int cuda_status(cudaError_t e, const char *what);
+// cudaMalloc for the library's own memory: when the device has none left, the
+// transposed levels that batches hold to be faster go back first (acfd_api.cu)
+cudaError_t device_malloc_bytes(void **p, size_t bytes);
+template <typename T>
+inline cudaError_t device_malloc(T **p, size_t bytes)
+{
+    return device_malloc_bytes(reinterpret_cast<void **>(p), bytes);
+}
 
 #define ACFD_CUDA(call)                                           \
     do {                                                          \

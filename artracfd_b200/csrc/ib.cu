@@ -1214,7 +1214,7 @@ unsigned blocks_for(long long n, int bs)
 int ib_create(IbState **out)
 {
     IbState *ib = new IbState();
-    cudaError_t e = cudaMalloc(&ib->status, sizeof(int));
+    cudaError_t e = device_malloc(&ib->status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ib->status, 0, sizeof(int));
     if (e != cudaSuccess) {
         delete ib;
@@ -1433,7 +1433,7 @@ int ib_upload(IbState *ib, const acfd_polyhedron_t *poly, int totN, const acfd_p
             set_error("acfd_geo_upload: missing geometry array");
             return ACFD_ERR_ARG;
         }
-        ACFD_CUDA(cudaMalloc(dst, bytes));
+        ACFD_CUDA(device_malloc(dst, bytes));
         ib->buffers.push_back(*dst);
         ACFD_CUDA(cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice));
         return ACFD_OK;
@@ -1452,7 +1452,7 @@ int ib_upload(IbState *ib, const acfd_polyhedron_t *poly, int totN, const acfd_p
             if ((st2 = dcopy(P.Ne, sizeof(double) * 3 * P.edgeN, &Ne)) != ACFD_OK) return st2;
             if ((st2 = dcopy(P.v, sizeof(double) * 3 * P.vertN, &v)) != ACFD_OK) return st2;
             if ((st2 = dcopy(P.Nv, sizeof(double) * 3 * P.vertN, &Nv)) != ACFD_OK) return st2;
-            ACFD_CUDA(cudaMalloc(&tri, sizeof(double) * 9 * P.faceN));
+            ACFD_CUDA(device_malloc(&tri, sizeof(double) * 9 * P.faceN));
             ib->buffers.push_back(tri);
             build_tri<<<blocks_for(P.faceN, 128), 128>>>((const int *)f, (const double *)v, (double *)tri, P.faceN);
             ACFD_CUDA(cudaGetLastError());
@@ -1465,7 +1465,7 @@ int ib_upload(IbState *ib, const acfd_polyhedron_t *poly, int totN, const acfd_p
             B.tri = (const double *)tri;
         }
     }
-    ACFD_CUDA(cudaMalloc(&ib->dev, sizeof(DevBody) * totN));
+    ACFD_CUDA(device_malloc(&ib->dev, sizeof(DevBody) * totN));
     ACFD_CUDA(cudaMemcpy(ib->dev, ib->host.data(), sizeof(DevBody) * totN, cudaMemcpyHostToDevice));
     // ghost lists, one per layer: a node is listed at most once, so the
     // smaller of the bodies' node boxes and the computed nodes bounds each
@@ -1485,15 +1485,15 @@ int ib_upload(IbState *ib, const acfd_polyhedron_t *poly, int totN, const acfd_p
     }
     void *gl_buf = nullptr, *cnt = nullptr;
     const int layers = std::max(1, part.gl);
-    ACFD_CUDA(cudaMalloc(&gl_buf, sizeof(int4) * (size_t)cap * layers));
+    ACFD_CUDA(device_malloc(&gl_buf, sizeof(int4) * (size_t)cap * layers));
     ib->buffers.push_back(gl_buf);
-    ACFD_CUDA(cudaMalloc(&cnt, sizeof(int) * layers));
+    ACFD_CUDA(device_malloc(&cnt, sizeof(int) * layers));
     ib->buffers.push_back(cnt);
     ib->ghosts = (int4 *)gl_buf;
     ib->nghost = (int *)cnt;
     ib->ghost_cap = (int)cap;
     ib->ngroups = (totN + 7) / 8;
-    ACFD_CUDA(cudaMalloc(&ib->groups, sizeof(BoxList) * ib->ngroups));
+    ACFD_CUDA(device_malloc(&ib->groups, sizeof(BoxList) * ib->ngroups));
     ACFD_CUDA(cudaDeviceSynchronize());
     int rc = upload_groups(ib, part, st);
     if (rc != ACFD_OK) return rc;
@@ -1580,13 +1580,13 @@ static int solid_scratch(IbState *ib, const acfd_partition_t &part, std::vector<
     if (!ib->sf_off || ib->col_n != totN || off[totN] > ib->sf_cap) {
         ib_release_solid(ib);
         const long long cap = std::max(1LL, off[totN] + off[totN] / 4);
-        ACFD_CUDA(cudaMalloc(&ib->sf_terms, sizeof(double) * 10 * (size_t)cap));
-        ACFD_CUDA(cudaMalloc(&ib->sf_valid, (size_t)cap));
-        ACFD_CUDA(cudaMalloc(&ib->sf_off, sizeof(long long) * (totN + 1)));
-        ACFD_CUDA(cudaMalloc(&ib->sf_lid, sizeof(int) * totN));
-        ACFD_CUDA(cudaMalloc(&ib->sf_force, sizeof(double) * 9 * totN));
-        ACFD_CUDA(cudaMalloc(&ib->col_key, sizeof(unsigned long long) * totN * totN));
-        ACFD_CUDA(cudaMalloc(&ib->col_N, sizeof(int) * 3 * totN * totN));
+        ACFD_CUDA(device_malloc(&ib->sf_terms, sizeof(double) * 10 * (size_t)cap));
+        ACFD_CUDA(device_malloc(&ib->sf_valid, (size_t)cap));
+        ACFD_CUDA(device_malloc(&ib->sf_off, sizeof(long long) * (totN + 1)));
+        ACFD_CUDA(device_malloc(&ib->sf_lid, sizeof(int) * totN));
+        ACFD_CUDA(device_malloc(&ib->sf_force, sizeof(double) * 9 * totN));
+        ACFD_CUDA(device_malloc(&ib->col_key, sizeof(unsigned long long) * totN * totN));
+        ACFD_CUDA(device_malloc(&ib->col_N, sizeof(int) * 3 * totN * totN));
         ib->sf_cap = cap;
         ib->col_n = totN;
     }
@@ -1702,7 +1702,7 @@ int ib_transform(IbState *ib, int n, const double O[3], const double scale[3], c
                             {-Sy, Sx * Cy, Cx * Cy}};
     for (int a = 0; a < 3; ++a)
         for (int b = 0; b < 3; ++b) M.rot[a][b] = R[a][b];
-    if (!ib->motion_part) ACFD_CUDA(cudaMalloc(&ib->motion_part, sizeof(BoxPart) * kMotionBlocks));
+    if (!ib->motion_part) ACFD_CUDA(device_malloc(&ib->motion_part, sizeof(BoxPart) * kMotionBlocks));
     const long long total = 2LL * B.vertN + B.faceN + B.edgeN;
     const int nblk = (int)std::min<long long>(kMotionBlocks, (total + kMotionThreads - 1) / kMotionThreads);
     move_surface<<<nblk, kMotionThreads, 0, st>>>(M, const_cast<double *>(B.v), const_cast<double *>(B.Nf),
@@ -1794,7 +1794,7 @@ int ib_compute_geometric_field(IbState *ib, const Grid &g, const ModelParams &m,
     if (ib->joined_n < g.nn) {
         cudaFree(ib->joined);
         ib->joined = nullptr;
-        ACFD_CUDA(cudaMalloc(&ib->joined, (size_t)g.nn));
+        ACFD_CUDA(device_malloc(&ib->joined, (size_t)g.nn));
         ib->joined_n = g.nn;
     }
     const long long pin = (long long)(g.hi[0] - g.lo[0]) * (g.hi[1] - g.lo[1]) * (g.hi[2] - g.lo[2]);

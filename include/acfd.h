@@ -399,7 +399,14 @@ int acfd_mlp_adam(float *params, const float *grad, float *m, float *v, int step
  * immersed bodies. */
 typedef struct acfd_batch acfd_batch_t;
 /* Create a batch of ncase cases (parts[c], models[c]); each case gets its own
- * device state as acfd_init would allocate it. */
+ * device state as acfd_init would allocate it.  Where every case's ghost fill is
+ * copies and all are viscous or all inviscid, the batch also holds its states
+ * transposed (as much memory again) and runs the X half steps as Y sweeps of them,
+ * when that takes at most half of the free memory and a quarter of the device's.
+ * The library gives them back when one of its own allocations finds no memory; the
+ * batch then sweeps X directly.  The two agree to FP32 round-off, so the last bits
+ * of a batch depend on which it runs (acfd_batch_transposed); ACFD_X_TRANSPOSE=0 in
+ * the environment at the creation keeps the X sweep. */
 int acfd_batch_init(int ncase, const acfd_partition_t *parts, const acfd_model_t *models, acfd_batch_t **out);
 int acfd_batch_finalize(acfd_batch_t *b);
 /* The case handle of case c, for acfd_sync_to_device / acfd_sync_to_host /
@@ -432,6 +439,8 @@ int acfd_batch_set_kernel(acfd_batch_t *b, int kernel);
 /* Run the batch's work on the caller's CUDA stream (cudaStream_t as void*);
  * the library's own stream is released. */
 int acfd_batch_set_stream(acfd_batch_t *b, void *stream);
+/* 1 when the next step runs the X half steps on the transposed states. */
+int acfd_batch_transposed(acfd_batch_t *b, int *on);
 /* Kernels launched by the batch so far (graph replays count their kernel
  * nodes). */
 int acfd_batch_stats(acfd_batch_t *b, long long *launches);
