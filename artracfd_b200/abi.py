@@ -211,6 +211,7 @@ def load_library(path: str | None = None):
         "acfd_transform_polyhedron": [vp, i, dp, dp, dp, dp, dp, dp, dp],
         "acfd_geo_fetch": [vp, i, vp, vp, vp, vp],
         "acfd_weno_batch": [i, i, vp, vp, i],
+        "acfd_line_roots": [vp, vp, vp, i],
         "acfd_fhat_batch": [ctypes.POINTER(Model), i, i, vp, vp, i],
         "acfd_batch_init": [i, ctypes.POINTER(Partition), ctypes.POINTER(Model), pp],
         "acfd_batch_finalize": [vp],

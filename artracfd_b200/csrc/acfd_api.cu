@@ -58,6 +58,7 @@ int launch_stage_plane_fp32(const Grid &, const ModelParams &, const StageArgs &
                             const PlaneTile &, const CUtensorMap &, cudaStream_t);
 int launch_stage_line(const Grid &, const ModelParams &, const StageArgs &, int, bool, const LineTile &,
                       const CUtensorMap &, const CUtensorMap &, cudaStream_t);
+int launch_line_roots(const double *, double *, double *, int, cudaStream_t);
 int launch_weno_batch_exact(int, const double *, double *, int, cudaStream_t);
 int launch_weno_batch_fast(int, const double *, double *, int, cudaStream_t);
 int launch_weno_batch_fp32(int, const double *, double *, int, cudaStream_t);
@@ -2497,6 +2498,25 @@ int acfd_weno_batch(int scheme, int mode, const double *F, double *Fhat, int cou
     }
     cudaFree(dF);
     cudaFree(dO);
+    return st;
+}
+
+int acfd_line_roots(const double *x, double *rsqrt, double *rcp, int count)
+{
+    if (!x || !rsqrt || !rcp || count < 0) {
+        set_error("acfd_line_roots: bad arguments");
+        return ACFD_ERR_ARG;
+    }
+    const size_t bytes = sizeof(double) * (size_t)count;
+    double *d = nullptr;  // x, then the two results
+    ACFD_CUDA(device_malloc(&d, 3 * bytes + 8));
+    cudaError_t e = cudaMemcpy(d, x, bytes, cudaMemcpyHostToDevice);
+    int st = e == cudaSuccess ? launch_line_roots(d, d + count, d + 2 * (size_t)count, count, 0) : cuda_status(e, "cudaMemcpy");
+    if (st == ACFD_OK && ((e = cudaMemcpy(rsqrt, d + count, bytes, cudaMemcpyDeviceToHost)) != cudaSuccess ||
+                          (e = cudaMemcpy(rcp, d + 2 * (size_t)count, bytes, cudaMemcpyDeviceToHost)) != cudaSuccess)) {
+        st = cuda_status(e, "cudaMemcpy");
+    }
+    cudaFree(d);
     return st;
 }
 

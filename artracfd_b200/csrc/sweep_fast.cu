@@ -58,4 +58,12 @@ int launch_stage_line(const Grid &g, const ModelParams &m, const StageArgs &a, i
     return form_fast::launch_line_impl(g, m, a, s, viscous, lt, map, omap, st);
 }
 
+int launch_line_roots(const double *x, double *rsqrt, double *rcp, int count, cudaStream_t st)
+{
+    if (count <= 0) return ACFD_OK;
+    form_fast::line::roots<<<(unsigned)((count + 255LL) / 256), 256, 0, st>>>(x, rsqrt, rcp, count);
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? ACFD_OK : cuda_status(e, "line roots launch");
+}
+
 }  // namespace acfd

@@ -45,9 +45,14 @@ namespace ACFD_NS {
 
 namespace line {
 
-// 1/sqrt(x) for positive normal x: the hardware approximation y (relative
-// error e0 < 2^-22) and one step of the third-order iteration
-// y (1 + e/2 + 3/8 e^2), e = 1 - x y^2, whose relative error is 5/16 e^3.
+// 1/sqrt(x) for positive normal x, from the hardware's approximation y by one step
+// of the third-order iteration of Householder's family (A. S. Householder, The
+// Numerical Treatment of a Single Nonlinear Equation, 1970): the binomial series
+// of y (1 - e)^(-1/2), e = 1 - x y^2, up to e^2.  The instruction works in the
+// 1.11.20 format, its result's lower 32 bits are zero: |d| < 2^-20 relative.  With
+// e = -2 d the step leaves 5/16 |e|^3 < 2^-58, below the roundings: of x y into e
+// (2^-54 in the result) and of the result (2^-53), 1.5 x 2^-53 in all
+// (tests/test_gpu_line_roots.py).
 __device__ __forceinline__ double rsqrt3(double x)
 {
     double y;
@@ -56,8 +61,9 @@ __device__ __forceinline__ double rsqrt3(double x)
     return fma(fma(0.375, e, 0.5), __dmul_rn(y, e), y);
 }
 
-// 1/x for normal x: the hardware approximation and one third-order step
-// y (1 + e + e^2), e = 1 - x y
+// 1/x for normal x and 1/x, the same way: the geometric series of y / (1 - e),
+// e = 1 - x y (one rounding, of |e| < 2^-20), up to e^2; it leaves |e|^3 < 2^-60
+// beside the result's rounding, 1.01 x 2^-53 in all.
 __device__ __forceinline__ double rcp3(double x)
 {
     double y;
@@ -308,6 +314,15 @@ __device__ __forceinline__ void viscous_part(const Gas &k, const Node &c, const 
     Fv[2] = t2;
     const double w = fma(t0, c.u + n.u, fma(ts, c.v + n.v, t2 * (c.w + n.w)));
     Fv[3] = fma(k.heat * mu, (n.T - c.T) * k.dds, 0.5 * w);
+}
+
+// rsqrt3 and rcp3 of count values (acfd_line_roots)
+__global__ void roots(const double *x, double *rsqrt, double *rcp, int count)
+{
+    const int q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= count) return;
+    rsqrt[q] = rsqrt3(x[q]);
+    rcp[q] = rcp3(x[q]);
 }
 
 }  // namespace line

@@ -455,6 +455,9 @@ int acfd_weno_batch(int scheme, int mode, const double *F, double *Fhat, int cou
  * first 4), Fhat count x 5. */
 int acfd_fhat_batch(const acfd_model_t *model, int s, int mode, const double *Ust,
         double *Fhat, int count);
+/* 1/sqrt(x) and 1/x of count positive values as the FP64 line-march stages
+ * compute them (no reference counterpart; for their error bounds). */
+int acfd_line_roots(const double *x, double *rsqrt, double *rcp, int count);
 
 #ifdef __cplusplus
 }
