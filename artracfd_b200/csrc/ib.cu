@@ -357,9 +357,6 @@ __device__ __forceinline__ void add_weighted(const double Uoh[6], double tiny, d
     wsum = wsum + w;
 }
 
-// inverse distance weighting (immersed_boundary.c:413-473); type TYPED: fluid
-// nodes, TYPEF: fluid nodes that were fluid before this mapping (not joined),
-// r >= 1: nodes of body did in ghost layer r
 __device__ void orthogonal_space(const double N[3], double Ta[3], double Tb[3])
 {
     int mark = 2;
@@ -420,17 +417,18 @@ __global__ void ib_list(IbGrid G, const BoxList *groups, int gidx, const int *fl
 constexpr int kGhostWarps = 4;    // warps per block of ib_ghost
 constexpr int kIdwBatch = 4;      // candidates per lane evaluated before the ordered sum
 
-// Inverse distance weighting by one warp (the candidates of the serial
-// version's k, j, i loop order, 32 x kIdwBatch at a time).  Every lane
-// evaluates candidates; those that qualify write w and Uoh[n] * w to the warp's
+// Inverse distance weighting (immersed_boundary.c:413-473) by one warp, over the
+// nodes of a type: kTypeD fluid nodes, kTypeF fluid nodes that were fluid before
+// this mapping (not joined), r >= 1 nodes of body did in ghost layer r.  The
+// candidates come in the reference's k, j, i loop order, 32 x kIdwBatch at a time.
+// Every lane evaluates candidates; those that qualify write w and Uoh[n] * w to the warp's
 // shared scratch at their rank, one row per sum, and lanes 0..6 add their row in
-// that order (Uo[0..5], wsum), so every sum takes exactly the serial version's
+// that order (Uo[0..5], wsum), so every sum takes exactly the reference's
 // additions in the same order.  All lanes return the same values.  The rows are
 // read ahead of the additions, whose chain (eight cycles a term) is then what a
 // sum costs: with the terms found one by one through the bits of the ballots,
 // and 64-bit divisions for the candidates' offsets, a layer of the ghost nodes
 // of eight spheres (5,200 nodes) took 17.1 us, 14.7 now.
-// joined (type kTypeF only): nodes left out.
 constexpr int kIdwRow = 32 * kIdwBatch + 5;  // doubles between the rows of the scratch (odd: no bank conflicts)
 
 __device__ double idw_warp(const IbGrid &G, const ModelParams &mp, const double *U, const int *flags,
