@@ -939,8 +939,9 @@ __device__ __forceinline__ int layer_of(const IbGrid &G, int q)
     return 0;
 }
 
-// interfacial layer, ghost layer and the joined mark (SetInterfacialField)
-__global__ void map_interface(IbGrid G, int *flags, unsigned char *joined)
+// interfacial layer, ghost layer and the joined mark (SetInterfacialField); the
+// joined nodes also go to a list (its first cap nodes, in any order; all counted)
+__global__ void map_interface(IbGrid G, int *flags, unsigned char *joined, int4 *list, int *njoined, long long cap)
 {
     const Grid &g = G.g;
     int i, j, k;
@@ -948,7 +949,12 @@ __global__ void map_interface(IbGrid G, int *flags, unsigned char *joined)
     const long long nn = g.nn;
     const long long id = node_of(g, i, j, k);
     const int did = flags[id];
-    joined[id] = (flags[3 * nn + id] != did && did == 0) ? 1 : 0;
+    const bool join = flags[3 * nn + id] != did && did == 0;
+    joined[id] = join ? 1 : 0;
+    if (join) {
+        const int slot = atomicAdd(njoined, 1);
+        if (slot < cap) list[slot] = make_int4(i, j, k, 0);
+    }
     int lid = 0, gst = 0;
     if (did != 0) {
         for (int q = 0; q < G.pathSep[0]; ++q) {
@@ -974,19 +980,53 @@ __global__ void map_interface(IbGrid G, int *flags, unsigned char *joined)
     flags[3 * nn + id] = gst;
 }
 
-// refill newly uncovered fluid nodes from fluid nodes that stayed fluid: a thread
-// looks at a node, and the warp reconstructs the few that joined one after the
-// other (a thread per node searched its box alone: 105 us at 192^3 with eight
-// moving spheres, 48 now)
+// a newly uncovered fluid node from the fluid nodes that stayed fluid, by a warp
+__device__ void refill_node(const IbGrid &G, const ModelParams &mp, double *U, int *flags, const unsigned char *joined,
+                            const int c[3], double *scratch, int *status)
+{
+    const long long nn = G.g.nn, id = node_of(G.g, c[0], c[1], c[2]);
+    double p[3], Uo[6];
+    node_point(G, c[2], c[1], c[0], p);
+    const double ws = idw_warp(G, mp, U, flags, joined, c, p, kIbR, kTypeF, 0, Uo, scratch, status);
+    for (int v = 0; v < 6; ++v) Uo[v] = Uo[v] / ws;
+    Uo[0] = Uo[4] / (Uo[5] * mp.gasR);
+    double Uc[5];
+    to_conservative(mp.gamma, Uo, Uc);
+    if ((threadIdx.x & 31) == 0) {
+        for (int v = 0; v < 5; ++v) U[v * nn + id] = Uc[v];
+        flags[nn + id] = -1;
+    }
+}
+
+// Refill of the newly uncovered fluid nodes, a warp per node of map_interface's
+// list, so that the nodes that a flat face uncovers, whole rows of them, spread
+// over the chip.  ComputeGeometricField on 129^3 nodes with a thread per node, with
+// warps that take the nodes of their own rows, and with the list, us: a flat face
+// that moves by 0.9 cells along z 353, 1,470 and 307, along x 1,052, 512 and 383; a
+// sphere of 40 cells' radius along z 452, 713 and 286; one of 10 cells' 203, 197 and
+// 87.  Without room for all of them in the list (a large body taken away) a warp
+// looks for them among kRefillNodes nodes a thread and takes them one after the
+// other.
 constexpr int kRefillNodes = 8;
 __global__ void __launch_bounds__(kGhostWarps * 32) map_refill(IbGrid G, ModelParams mp, double *U, int *flags,
-                                                               const unsigned char *joined, int *status)
+                                                               const unsigned char *joined, const int4 *list,
+                                                               const int *njoined, long long cap, int *status)
 {
     __shared__ double scratch[kGhostWarps][7 * kIdwRow];
+    double *sp = scratch[threadIdx.x >> 5];
     const Grid &g = G.g;
     const int lane = threadIdx.x & 31;
-    const long long nn = g.nn;
-    // kRefillNodes nodes a thread, their marks loaded together (bit q of marks)
+    const int count = *njoined;
+    if (count <= cap) {
+        for (long long w = (long long)blockIdx.x * kGhostWarps + (threadIdx.x >> 5); w < count;
+             w += (long long)gridDim.x * kGhostWarps) {
+            const int4 q = list[w];
+            const int c[3] = {q.x, q.y, q.z};
+            refill_node(G, mp, U, flags, joined, c, sp, status);
+        }
+        return;
+    }
+    // the marks of a thread's nodes loaded together (bit q of marks)
     const long long first = (long long)blockIdx.x * kRefillNodes * blockDim.x + (threadIdx.x & ~31);
     unsigned marks = 0;
 #pragma unroll
@@ -1001,19 +1041,7 @@ __global__ void __launch_bounds__(kGhostWarps * 32) map_refill(IbGrid G, ModelPa
         for (unsigned m = __ballot_sync(0xffffffffu, marks >> q & 1u); m; m &= m - 1) {
             int c[3];
             pin_node(g, first + (long long)q * blockDim.x + __ffs(m) - 1, c[0], c[1], c[2]);
-            const long long id = node_of(g, c[0], c[1], c[2]);
-            double p[3], Uo[6];
-            node_point(G, c[2], c[1], c[0], p);
-            const double ws = idw_warp(G, mp, U, flags, joined, c, p, kIbR, kTypeF, 0, Uo, scratch[threadIdx.x >> 5],
-                                       status);
-            for (int v = 0; v < 6; ++v) Uo[v] = Uo[v] / ws;
-            Uo[0] = Uo[4] / (Uo[5] * mp.gasR);
-            double Uc[5];
-            to_conservative(mp.gamma, Uo, Uc);
-            if (lane == 0) {
-                for (int v = 0; v < 5; ++v) U[v * nn + id] = Uc[v];
-                flags[nn + id] = -1;
-            }
+            refill_node(G, mp, U, flags, joined, c, sp, status);
         }
     }
 }
@@ -1821,9 +1849,16 @@ int ib_compute_geometric_field(IbState *ib, const Grid &g, const ModelParams &m,
         map_body<<<blocks, kMapThreads, smem, st>>>(G, ib->dev, n, bl, flags, ib->status);
         ACFD_CUDA(cudaGetLastError());
     }
-    map_interface<<<blocks_for(pin, 256), 256, 0, st>>>(G, flags, ib->joined);
+    // the list of joined nodes lies in the ghost list, which is built again below
+    const long long cap = (long long)ib->ghost_cap * std::max(1, part.gl);
+    ACFD_CUDA(cudaMemsetAsync(ib->nghost, 0, sizeof(int), st));
+    map_interface<<<blocks_for(pin, 256), 256, 0, st>>>(G, flags, ib->joined, ib->ghosts, ib->nghost, cap);
     ACFD_CUDA(cudaGetLastError());
-    map_refill<<<blocks_for(pin, kGhostWarps * 32 * kRefillNodes), kGhostWarps * 32, 0, st>>>(G, m, U, flags, ib->joined, ib->status);
+    // blocks for the scan of all nodes, and enough warps for the list on small grids
+    const long long blocks = std::max<long long>(blocks_for(pin, kGhostWarps * 32 * kRefillNodes),
+                                                 std::min<long long>(blocks_for(pin, kGhostWarps), 148LL * 12));
+    map_refill<<<(unsigned)blocks, kGhostWarps * 32, 0, st>>>(G, m, U, flags, ib->joined, ib->ghosts, ib->nghost, cap,
+                                                              ib->status);
     ACFD_CUDA(cudaGetLastError());
     if (part.gl >= 1) {
         const int rc = build_lists(ib, G, part, flags, st);
