@@ -422,8 +422,9 @@ int encode_state_maps(acfd_case *cs)
 // (line_iterations), in segments or in shares, cost less than the brick's tiles of
 // 240 nodes: an iteration of one consumer warp on every SM takes as long as the
 // chip needs for 14 to 15 tiles (inviscid: 2.3-2.4 us against 13 ns a tile and
-// twelve warps) or 13.5 (viscous: 2.0-2.8 us, 17.5 ns, eight or twelve warps); the
-// rule says 14 and 12, the brick's last wave being the fuller one.  Grids that
+// twelve warps) or 13.5 (viscous: 2.0-2.8 us, 17.5 ns, eight or twelve warps).  The
+// rule says 14 and 11, which cost least over the 76 shapes measured (the small ones
+// see partial waves of both).  Grids that
 // leave the march's lanes empty stay on the brick: steps on the line march and on
 // the brick, us, 512 x 512 cells in a plane 434 and 335, 1 x 200,000 x 1 cells
 // 18,270 and 1,450 (the march has one line); 700 x 300 x 2 cells 597 and 1,152.
@@ -451,7 +452,7 @@ void fp64_defaults(acfd_case *cs)
             tiles *= n;
             if (a > 0 && n > 65535) launchable = false;
         }
-        long long cost = std::min(seg, share) * line_shape(s == 0, visc).warps * (visc ? 12 : 14);  // in tiles
+        long long cost = std::min(seg, share) * line_shape(s == 0, visc).warps * (visc ? 11 : 14);  // in tiles
         if (cs->model.multidim == 1 && s != 0) cost = cost * 7 / 4;
         if (launchable && cost > tiles) continue;
         cs->tile_var[ACFD_FP64][s] = kPlaneFirst + (seg <= share ? 0 : 3);
